@@ -347,6 +347,9 @@ gnd_status gnd_gpu_scene_upload(gnd_gpu_ctx* ctxh, const gnd_scene_desc* d, gnd_
         }
         v.numEmitters = d->num_emitters;
         v.numInstances = d->num_instances;
+        v.hasCubes = 0;
+        for (int i = 0; i < d->num_instances; ++i)
+            if ((it[i].kind & ~kInstAnimated) == kShapeCube) v.hasCubes = 1;
         ds->numNodes = d->num_nodes;
         if (deviceBlas) {
             MeshTreeInput mi{};

@@ -115,6 +115,18 @@ __device__ __forceinline__ bool cubeTest(V3 ex, V3 o, V3 d, float tmin, float tm
     return true;
 }
 
+// True for a ray that can hit nothing although it enters every box: one with a NaN in its
+// origin or direction (a degenerate BSDF sample). A NaN slab term never excludes a child,
+// so such a ray would visit every node and triangle of the scene (4.8 s for one path of the
+// 5.2M-triangle sphere grid, ended by the iteration limit). The object-space ray has NaN in
+// every component of the one that held it; det or u of a triangle is then NaN and its
+// comparison false (mesh.cpp:259-291), and both roots of a sphere are NaN. A cube reports a
+// hit at tMax (its interval is never narrowed), which is accepted when finite.
+__device__ __forceinline__ bool missesAll(const SceneView& s, const TRay& r) {
+    const bool bad = isnan(r.o.x) || isnan(r.o.y) || isnan(r.o.z) || isnan(r.d.x) || isnan(r.d.y) || isnan(r.d.z);
+    return bad && !(s.hasCubes && r.tmax < 3.402823466e38f);
+}
+
 // World-to-object rows of animated instance `id` at `time` (primitive.cpp:49:
 // m_objectToWorld.interpolate(time).inverse()); r0..r2 hold the start transform's rows on
 // entry, which stay for time <= 0. Only the MOTION variants of the traversal call it
@@ -145,7 +157,7 @@ __device__ __forceinline__ int traceRay(const SceneView& s, const TRay& ray, THi
     hit.u = hit.v = 0.f;
     hit.inst = -1;
     hit.slot = 0xFFFFFFFFu;
-    if (s.tlasRoot == kEmpty) return kTraceOk;
+    if (s.tlasRoot == kEmpty || missesAll(s, ray)) return kTraceOk;
     const V3 wo = ray.o, wd = ray.d;
     const float wtmin = ray.tmin;
     float tmax = ray.tmax;          // shrinks with every accepted hit
@@ -613,7 +625,9 @@ __device__ __forceinline__ int persistentTrace(Src& src, uint32_t* fetchCounter,
             // a source may decline an item (it belongs to another kernel of the launch)
             if (src.load(idx, r, sv, nm)) {
                 travInit(t, *sv, r);
-                t.next = sv->tlasRoot;   // kEmpty for a scene without primitives
+                // kEmpty for a scene without primitives; the counting variants report what
+                // the traversal visits, a NaN ray's too
+                t.next = !COUNT && missesAll(*sv, r) ? kEmpty : sv->tlasRoot;
                 active = true;
                 iter = 0;
             }

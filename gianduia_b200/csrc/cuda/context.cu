@@ -109,7 +109,7 @@ constexpr uint32_t kNodeBadRef = 1u, kNodeBadLeaf = 2u, kNodeSlowBounds = 4u;
 
 // Checks every node of an uploaded tree: inner references below n, leaf ranges below
 // leafLimit (triangles or top-level entries), and whether the bounds allow the fast slab
-// test (no NaN, lo <= hi on every non-empty child).
+// test (no NaN, lo <= hi on every non-empty child, inf and -inf on the empty ones).
 __global__ void kValidateNodes(const Node4* __restrict__ nodes, int64_t n, int64_t leafLimit, uint32_t* flags) {
     uint32_t f = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -122,6 +122,8 @@ __global__ void kValidateNodes(const Node4* __restrict__ nodes, int64_t n, int64
                 if (isnan(lo[a]) || isnan(hi[a])) f |= kNodeSlowBounds;
                 if (r != kEmpty && !(lo[a] <= hi[a])) f |= kNodeSlowBounds;
             }
+            // an empty child is told by its bounds alone there
+            if (r == kEmpty && !(lo[0] == INFINITY && hi[0] == -INFINITY)) f |= kNodeSlowBounds;
             if (r == kEmpty) continue;
             if (!isLeaf(r)) {
                 if ((int64_t)r >= n) f |= kNodeBadRef;

@@ -126,11 +126,11 @@ struct Tune {
     int roundIters = 8;       // wavefront iterations per host round of a batched render
     int travBlocks = 8;       // persistent traversal blocks (128 threads) per SM
     int sort = 1;             // 1: classify hits and shade per material class
-    int smem = 32;            // traversal stack entries in shared memory (16 or 32)
+    int smem = 32;            // traversal stack in shared memory: 32: 16 entries, 16: 8 entries
     int graphs = 1;           // replay iteration pairs as CUDA graphs
     int sampleFilm = 1;       // batched box-filter renders: per-sample records, no film atomics
-    int specExtend = 0;       // speculative node traversal in the extend kernel
-    int specShadow = 0;       // speculative node traversal in the shadow kernel
+    int specExtend = 0;       // no effect
+    int specShadow = 0;       // no effect
     int raySort = 0;          // reorder each iteration's closest-hit queries by ray key
     int leafBatch = 32;       // closest-hit traversal of renders: lanes holding a leaf that end the node phase
     int traceLeafBatch = 12;  // the same for the scene's ray batches

@@ -26,12 +26,13 @@ struct BatchSrc {
     uint32_t* trisOut;
     TraceCounters* cnt;
     const uint32_t* perm;
+    uint32_t cur = 0;   // the ray in flight
     unsigned long long sumNodes = 0, sumTris = 0;   // COUNT: this lane's rays, for the context totals
     __device__ uint32_t count() const { return n; }
     __device__ bool load(uint32_t k, TRay& r, const SceneView*& s, const uint8_t*& nm) {
-        const uint32_t i = perm ? __ldg(perm + k) : k;
-        float4 a = __ldg(reinterpret_cast<const float4*>(rays + i));
-        float4 b = __ldg(reinterpret_cast<const float4*>(rays + i) + 1);
+        cur = perm ? __ldg(perm + k) : k;
+        const float4 a = __ldg(reinterpret_cast<const float4*>(rays + cur));
+        const float4 b = __ldg(reinterpret_cast<const float4*>(rays + cur) + 1);
         r.o = v3(a.x, a.y, a.z);
         r.tmin = a.w;
         r.d = v3(b.x, b.y, b.z);
@@ -41,8 +42,15 @@ struct BatchSrc {
         if (COUNT) { cnt->nodes = 0; cnt->tris = 0; }
         return true;
     }
-    __device__ void store(uint32_t k, const THit& h, const SceneView&) {
-        const uint32_t i = perm ? __ldg(perm + k) : k;
+    __device__ void world(V3& o, V3& d, float& tmin) const {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(rays + cur));
+        const float4 b = __ldg(reinterpret_cast<const float4*>(rays + cur) + 1);
+        o = v3(a.x, a.y, a.z);
+        tmin = a.w;
+        d = v3(b.x, b.y, b.z);
+    }
+    __device__ void store(uint32_t, const THit& h, const SceneView&) {
+        const uint32_t i = cur;
         if (COUNT) {
             nodesOut[i] = cnt->nodes;
             trisOut[i] = cnt->tris;
@@ -62,22 +70,21 @@ struct BatchSrc {
     }
 };
 
-// MINB: blocks per SM the kernel is compiled to fit (8: 64 registers; 9 and 10 trade
-// registers, some spilled, for more resident warps; gnd_tune trace_blocks).
-template <bool ANY, bool COUNT, int MINB = kTraceBlocksPerSM>
-__global__ void __launch_bounds__(kTraceBlock, MINB)
+template <bool ANY, bool COUNT>
+__global__ void __launch_bounds__(kTraceBlock, kTraceBlocksPerSM)
     traceKernel(const SceneView* __restrict__ sv, const gnd_ray* __restrict__ rays, uint32_t n, gnd_hit* __restrict__ hits,
                 uint8_t* __restrict__ occ, uint32_t* __restrict__ nodesOut, uint32_t* __restrict__ trisOut,
                 uint32_t* fetch, uint32_t* errWord, unsigned long long* totals, const uint32_t* __restrict__ perm,
                 uint32_t leafBatch) {
-    __shared__ uint32_t stack[kSmemStack * kTraceBlock];
+    __shared__ TEntry<!ANY> stack[kSmemStack * kTraceBlock];
+    __shared__ uint32_t map[kTraceBlock];
     TraceCounters cnt{0, 0, 0, 0, 0};
     BatchSrc<ANY, COUNT> src{sv, rays, n, hits, occ, nodesOut, trisOut, &cnt, perm};
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         atomicAdd(&totals[kTraceTotalRays], (unsigned long long)n);
         if (COUNT) atomicAdd(&totals[kTraceTotalCountedRays], (unsigned long long)n);
     }
-    int err = persistentTrace<kTraceBlock, ANY, COUNT>(src, fetch, stack, &cnt, leafBatch);
+    int err = persistentTrace<kTraceBlock, ANY, COUNT>(src, fetch, stack, map, &cnt, leafBatch);
     if (COUNT) {
         unsigned long long nn = src.sumNodes, nt = src.sumTris;
         for (int o = 16; o > 0; o >>= 1) {
@@ -134,9 +141,9 @@ void launchTrace(Context* c, DeviceScene& ds, const gnd_ray* dr, int64_t n, gnd_
                  uint32_t* dn, uint32_t* dt, cudaStream_t st) {
     if (n <= 0) return;
     if (n >= (int64_t)0xF0000000LL) throw Error(GND_ERR_INVALID, "ray batch too large (limit 4e9 rays per call)");
-    int64_t blocks = (n + kTraceBlock - 1) / kTraceBlock;
-    // the counting kernel always fits 8 blocks per SM
-    const int bps = dn ? kTraceBlocksPerSM : std::min(std::max(ds.tune.traceBlocks, 1), 10);
+    // small batches: a warp per ray as long as the grid has room (persistentTrace spreads them)
+    int64_t blocks = (n + kTraceBlock / 32 - 1) / (kTraceBlock / 32);
+    const int bps = std::min(std::max(ds.tune.traceBlocks, 1), kTraceBlocksPerSM);
     int g = (int)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)c->numSMs * bps));
     uint32_t* ew = c->errWord.as<uint32_t>();
     uint32_t* fetch = c->nextFetchCounter();
@@ -162,11 +169,7 @@ void launchTrace(Context* c, DeviceScene& ds, const gnd_ray* dr, int64_t n, gnd_
     }
     const uint32_t lb = (uint32_t)ds.tune.traceLeafBatch;
     if (dn) traceKernel<false, true><<<g, kTraceBlock, 0, st>>>(sv, dr, nn, nullptr, nullptr, dn, dt, fetch, ew, tot, order, lb);
-    else if (docc && bps == 9) traceKernel<true, false, 9><<<g, kTraceBlock, 0, st>>>(sv, dr, nn, nullptr, docc, nullptr, nullptr, fetch, ew, tot, order, lb);
-    else if (docc && bps == 10) traceKernel<true, false, 10><<<g, kTraceBlock, 0, st>>>(sv, dr, nn, nullptr, docc, nullptr, nullptr, fetch, ew, tot, order, lb);
     else if (docc) traceKernel<true, false><<<g, kTraceBlock, 0, st>>>(sv, dr, nn, nullptr, docc, nullptr, nullptr, fetch, ew, tot, order, lb);
-    else if (bps == 9) traceKernel<false, false, 9><<<g, kTraceBlock, 0, st>>>(sv, dr, nn, dh, nullptr, nullptr, nullptr, fetch, ew, tot, order, lb);
-    else if (bps == 10) traceKernel<false, false, 10><<<g, kTraceBlock, 0, st>>>(sv, dr, nn, dh, nullptr, nullptr, nullptr, fetch, ew, tot, order, lb);
     else traceKernel<false, false><<<g, kTraceBlock, 0, st>>>(sv, dr, nn, dh, nullptr, nullptr, nullptr, fetch, ew, tot, order, lb);
     GND_CUDA(cudaGetLastError());
     c->counters.trace_batches += 1;
@@ -305,7 +308,7 @@ gnd_status gnd_gpu_trace_closest_fixed(gnd_gpu_ctx* ctxh, gnd_scene_id id, const
         cudaStream_t st = c->stream;
         GND_CUDA(cudaMemcpyAsync(dr, rays, sizeof(gnd_ray) * (size_t)n, cudaMemcpyHostToDevice, st));
         GND_CUDA(cudaMemsetAsync(fetch, 0, sizeof(uint32_t), st));
-        int64_t blocks = (n + kTraceBlock - 1) / kTraceBlock;
+        int64_t blocks = (n + kTraceBlock / 32 - 1) / (kTraceBlock / 32);
         int g = (int)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)c->numSMs * kTraceBlocksPerSM));
         traceKernel<false, false><<<g, kTraceBlock, 0, st>>>(ds.viewDev.as<SceneView>(), dr, (uint32_t)n, dh, nullptr,
                                                              nullptr, nullptr, fetch, c->errWord.as<uint32_t>(),

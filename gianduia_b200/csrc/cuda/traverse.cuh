@@ -145,14 +145,10 @@ __device__ __forceinline__ void animatedW2ORows(const SceneView& s, uint32_t id,
     r2 = make_float4(w.r[2][0], w.r[2][1], w.r[2][2], w.r[2][3]);
 }
 
-// Trace one ray. ANY: stop at the first hit (occlusion query). SKIP_NULL: ignore
-// instances whose material has no BSDF (index material) -- used by the path
-// integrator's shadow rays. COUNT: accumulate node visits and triangle tests.
-// `stk` points at this thread's first stack entry in shared memory; entries are
-// BLOCK apart. Returns an error bitmask (0 on success).
-template <int BLOCK, bool ANY, bool SKIP_NULL, bool COUNT, bool MOTION = false>
-__device__ __forceinline__ int traceRay(const SceneView& s, const TRay& ray, THit& hit, uint32_t* stk,
-                                        TraceCounters* cnt, const uint8_t* nullMask) {
+// Trace one ray to its closest hit. `stk` points at this thread's first stack entry in
+// shared memory; entries are BLOCK apart. Returns an error bitmask (0 on success).
+template <int BLOCK, bool MOTION = false>
+__device__ __forceinline__ int traceRay(const SceneView& s, const TRay& ray, THit& hit, uint32_t* stk) {
     hit.t = INFINITY;
     hit.u = hit.v = 0.f;
     hit.inst = -1;
@@ -184,7 +180,6 @@ __device__ __forceinline__ int traceRay(const SceneView& s, const TRay& ray, THi
         }
         if (!isLeaf(e)) {
             const Node4* nd = s.nodes + e;
-            if (COUNT) cnt->nodes++;
             float4 lx = ldg4(nd->lox), hx = ldg4(nd->hix), ly = ldg4(nd->loy);
             float4 hy = ldg4(nd->hiy), lz = ldg4(nd->loz), hz = ldg4(nd->hiz);
             uint4 ch = ldgu4(nd->child);
@@ -227,9 +222,7 @@ __device__ __forceinline__ int traceRay(const SceneView& s, const TRay& ray, THi
             for (uint32_t k = 0; k < count; ++k) {
                 float t, u, v;
                 uint32_t prim;
-                if (COUNT) cnt->tris++;
                 if (triTest(s.tris + first + k, o, d, tmin, tmax, t, u, v, prim)) {
-                    if (ANY) { hit.t = t; hit.inst = curInst; hit.slot = first + k; return err; }
                     tmax = t;
                     bestT = t;
                     hit.t = t; hit.u = u; hit.v = v;
@@ -242,7 +235,6 @@ __device__ __forceinline__ int traceRay(const SceneView& s, const TRay& ray, THi
         // top level: instances tlasList[first .. first + count)
         for (uint32_t k = 0; k < count; ++k) {
             uint32_t id = __ldg(s.tlasList + first + k);
-            if (SKIP_NULL && nullMask && nullMask[id]) continue;
             const InstTrav* it = s.instT + id;
             float4 r0 = ldg4(&it->w2o.r[0][0]), r1 = ldg4(&it->w2o.r[1][0]), r2 = ldg4(&it->w2o.r[2][0]);
             float4 meta = ldg4(&it->kind);
@@ -283,7 +275,6 @@ __device__ __forceinline__ int traceRay(const SceneView& s, const TRay& ray, THi
                 h = cubeTest(v3(meta.z, meta.w, ez), lo, ld, kEpsilon, tmax, th);
             }
             if (h && th < bestT) {
-                if (ANY) { hit.t = th; hit.inst = (int)id; return err; }
                 tmax = th;
                 bestT = th;
                 hit.t = th; hit.u = 0.f; hit.v = 0.f;
@@ -299,39 +290,60 @@ __device__ __forceinline__ int traceRay(const SceneView& s, const TRay& ray, THi
 // ---------------------------------------------------------------- persistent traversal
 // The same traversal as traceRay, restated as an incremental per-lane state machine for
 // persistent warps: lanes that finish a ray fetch the next one (warp-aggregated atomic on
-// a per-launch counter), and each round runs a node phase (every lane pops and tests
-// inner nodes until it holds a leaf) followed by a leaf phase (one primitive per step),
-// so the warp executes one code path at a time. Stack entries 0 .. SMEM-1 live in shared
-// memory and deeper ones in a per-lane local array (SMEM is a template parameter, 32 by
-// default), so shallow stacks never leave shared memory.
-constexpr int kSmemStack = 32;
+// a per-launch counter), and each round runs a node phase (every lane tests inner nodes
+// until it holds a leaf) and a leaf pass (the warp's lanes share out the pending triangles),
+// so the warp executes one code path at a time.
+//
+// What bounds it: instructions issued for the lanes that still have work (about 12 of 32 on
+// random rays), not bytes. Hence packed fp32 arithmetic for the slabs, a child entered or
+// popped in the same step as the test before it, children dropped at the pop when a hit
+// found meanwhile is nearer, and triangles of all lanes tested side by side.
+constexpr int kSmemStack = 16;
 constexpr int kPStackMax = 128;   // entries per ray, shared + local
 
-struct Trav {
-    V3 wo, wd;          // world ray
-    float time;         // shutter time (animated instances)
-    V3 o, d, inv;       // current ray (world, or object space inside a bottom-level tree)
-    float wtmin, tmin, tmax, bestT;
-    int curInst;
-    int sp;
-    bool fast, wfast;   // current / world ray: nodeKeysFast applies (see there)
-    uint32_t next;      // entry to visit next without a stack round trip, kEmpty when none
-    uint32_t leaf;      // pending primitives (a leaf reference advanced past those done), kEmpty when none
-    THit hit;           // t unused: a hit's distance is bestT (travHit)
+// Stack entry: a child reference and, for closest-hit queries, its visit key (entry
+// distance, see packKey; 0 for entries that are always taken).
+template <bool KEYED>
+struct TEntry;
+template <>
+struct TEntry<true> {
+    uint32_t ref, key;
+};
+template <>
+struct TEntry<false> {
+    uint32_t ref;
 };
 
-// SMEM: entries kept in shared memory (the block's array holds SMEM * BLOCK words); the
-// remaining kPStackMax - SMEM entries live in a per-lane local array.
-template <int BLOCK, int SMEM = kSmemStack>
+// SMEM: entries kept in shared memory (the block's array holds SMEM * BLOCK entries, entry k
+// of thread t at [k * BLOCK + t]: bank-conflict free); the remaining kPStackMax - SMEM live
+// in a per-lane local array.
+template <int BLOCK, int SMEM, bool KEYED>
 struct TStack {
     static_assert(SMEM > 0 && SMEM < kPStackMax, "shared part of the stack out of range");
-    uint32_t* smem;                 // this lane's column in the block's shared array
-    uint32_t local[kPStackMax - SMEM];
-    __device__ __forceinline__ void put(int k, uint32_t v) {
-        if (k < SMEM) smem[k * BLOCK] = v;
-        else local[k - SMEM] = v;
+    using Entry = TEntry<KEYED>;
+    Entry* smem;                 // this lane's column in the block's shared array
+    Entry local[kPStackMax - SMEM];
+    __device__ __forceinline__ void put(int k, uint32_t ref, uint32_t key) {
+        Entry e;
+        e.ref = ref;
+        if constexpr (KEYED) e.key = key;
+        if (k < SMEM) smem[k * BLOCK] = e;
+        else local[k - SMEM] = e;
     }
-    __device__ __forceinline__ uint32_t get(int k) const { return k < SMEM ? smem[k * BLOCK] : local[k - SMEM]; }
+    __device__ __forceinline__ Entry get(int k) const { return k < SMEM ? smem[k * BLOCK] : local[k - SMEM]; }
+};
+
+struct Trav {
+    V3 o, d, inv;       // current ray (world, or object space inside a bottom-level tree)
+    float tmin, tmax;   // tmax: the ray's, then the nearest hit's distance
+    int curInst;        // -1 at the top level
+    int sp;
+    uint32_t cur;       // inner node to test, kEmpty when none
+    uint32_t leaf;      // pending primitives (a leaf reference advanced past those done), kEmpty when none
+    bool fast, wfast;   // current / world ray: nodeKeysFast applies (see there)
+    float u, v;         // hit
+    int32_t inst;
+    uint32_t slot;
 };
 
 // True when (bound - o) * inv cannot be NaN for any finite or infinite node bound: the
@@ -343,18 +355,17 @@ __device__ __forceinline__ bool slabFinite(const SceneView& s, V3 o, V3 inv) {
 }
 
 __device__ __forceinline__ void travInit(Trav& t, const SceneView& s, const TRay& ray) {
-    t.wo = ray.o; t.wd = ray.d;
     t.o = ray.o; t.d = ray.d;
     t.inv = v3(__frcp_rn(ray.d.x), __frcp_rn(ray.d.y), __frcp_rn(ray.d.z));
     t.fast = t.wfast = slabFinite(s, t.o, t.inv) && !isnan(ray.tmin) && !isnan(ray.tmax);
-    t.wtmin = ray.tmin; t.tmin = ray.tmin; t.tmax = ray.tmax;
-    t.time = ray.time;
-    t.bestT = 3.402823466e38f;
+    t.tmin = ray.tmin; t.tmax = ray.tmax;
     t.curInst = -1;
     t.leaf = kEmpty;
-    t.next = kEmpty;
-    t.hit.t = INFINITY; t.hit.u = t.hit.v = 0.f; t.hit.inst = -1; t.hit.slot = 0xFFFFFFFFu;
     t.sp = 0;
+    t.u = t.v = 0.0f;
+    t.inst = -1;
+    t.slot = 0xFFFFFFFFu;
+    t.cur = s.tlasRoot;   // kEmpty for a scene without primitives
 }
 
 // Visit-order key of a hit child: the entry distance's bits with the child slot in the
@@ -366,11 +377,22 @@ constexpr uint32_t kMissKey = 0xFFFFFFFFu;
 __device__ __forceinline__ uint32_t packKey(float a, int slot) {
     return (__float_as_uint(a) & 0x7FFFFFFCu) | (uint32_t)slot;
 }
+// Stack entries with a key above this are beyond the nearest hit: no child of theirs would
+// be entered (its entry distance is no smaller), so they are dropped. The distance is widened
+// by far more than the rounding of a triangle's t, so that a leaf whose box lies a few ulp
+// beyond its own triangle is not. Keys are distances only when no entry distance can be
+// negative (tMin >= 0), tMax is a positive number and the slab test is the plain one (a NaN
+// term of the exact one may leave an infinite entry distance); otherwise everything is kept.
+__device__ __forceinline__ uint32_t cullKey(const Trav& t) {
+    return t.fast && t.tmin >= 0.0f && t.tmax > 0.0f ? __float_as_uint(t.tmax * (1.0f + 1.0f / 32768.0f)) : kMissKey;
+}
 
 // Child entry distances of one node for the current ray (bvhTraversal.h:57-72) as visit
 // keys; kMissKey for a missed or empty child. nodeKeysExact is the reference's lane arithmetic with
 // SSE min/max (the second operand when either is NaN), for any ray and any bounds.
-__device__ __forceinline__ void nodeKeysExact(const Node4* nd, const Trav& t, const uint32_t ref[4], uint32_t key[4]) {
+__device__ __forceinline__ void nodeKeysExact(const Node4* nd, const Trav& t, uint32_t key[4]) {
+    const uint4 ch = ldgu4(nd->child);
+    const uint32_t ref[4] = {ch.x, ch.y, ch.z, ch.w};
     float4 lx = ldg4(nd->lox), hx = ldg4(nd->hix);
     float t1[4] = {(lx.x - t.o.x) * t.inv.x, (lx.y - t.o.x) * t.inv.x, (lx.z - t.o.x) * t.inv.x, (lx.w - t.o.x) * t.inv.x};
     float t2[4] = {(hx.x - t.o.x) * t.inv.x, (hx.y - t.o.x) * t.inv.x, (hx.z - t.o.x) * t.inv.x, (hx.w - t.o.x) * t.inv.x};
@@ -397,80 +419,139 @@ __device__ __forceinline__ void nodeKeysExact(const Node4* nd, const Trav& t, co
     }
 }
 
+// Two fp32 operations per instruction (sm_100), each rounded as its scalar form is.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(uint64_t r, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(r)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// (bound - o) * inv of four bounds
+__device__ __forceinline__ void slab4(float4 b, uint64_t no, uint64_t iv, float t[4]) {
+    unpack2(mul2(add2(pack2(b.x, b.y), no), iv), t[0], t[1]);
+    unpack2(mul2(add2(pack2(b.z, b.w), no), iv), t[2], t[3]);
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 // The same distances with less work, for rays and nodes where it gives the same values
-// (t.fast: finite origin, finite non-zero inverse direction; fastBoxes: no NaN bound and
-// lo <= hi for every non-empty child). Then no slab term is NaN, so min/max are the
-// hardware ones, and because (bound - o) * inv is monotone in the bound, the smaller of
-// the two planes of an axis is the lo plane when inv > 0 and the hi plane when inv < 0:
-// the near and far planes are chosen once per axis from the direction's sign instead of
-// by a min/max per child. Empty children (ref kEmpty) are discarded as before. The
+// (t.fast: finite origin, finite non-zero inverse direction; fastBoxes: no NaN bound, lo <= hi
+// for every non-empty child, and lo = inf, hi = -inf for an empty one). Then no slab term is
+// NaN, so min/max are the hardware ones, and because (bound - o) * inv is monotone in the
+// bound, the smaller of the two planes of an axis is the lo plane when inv > 0 and the hi
+// plane when inv < 0: the near and far planes are chosen once per axis from the direction's
+// sign instead of by a min/max per child. An empty child has near = inf > far = -inf. The
 // result may differ from nodeKeysExact only in the sign of a zero key, which no
 // comparison sees.
-__device__ __forceinline__ void nodeKeysFast(const Node4* nd, const Trav& t, const uint32_t ref[4], uint32_t key[4]) {
+__device__ __forceinline__ void nodeKeysFast(const Node4* nd, const Trav& t, uint32_t key[4]) {
     const bool sx = t.inv.x < 0.0f, sy = t.inv.y < 0.0f, sz = t.inv.z < 0.0f;
     const float4 nx = ldg4(sx ? nd->hix : nd->lox), fx = ldg4(sx ? nd->lox : nd->hix);
     const float4 ny = ldg4(sy ? nd->hiy : nd->loy), fy = ldg4(sy ? nd->loy : nd->hiy);
     const float4 nz = ldg4(sz ? nd->hiz : nd->loz), fz = ldg4(sz ? nd->loz : nd->hiz);
-    const float n0[4] = {nx.x, nx.y, nx.z, nx.w}, f0[4] = {fx.x, fx.y, fx.z, fx.w};
-    const float n1[4] = {ny.x, ny.y, ny.z, ny.w}, f1[4] = {fy.x, fy.y, fy.z, fy.w};
-    const float n2[4] = {nz.x, nz.y, nz.z, nz.w}, f2[4] = {fz.x, fz.y, fz.z, fz.w};
+    float n0[4], f0[4], n1[4], f1[4], n2[4], f2[4];
+    {
+        const uint64_t no = pack2(-t.o.x, -t.o.x), iv = pack2(t.inv.x, t.inv.x);
+        slab4(nx, no, iv, n0);
+        slab4(fx, no, iv, f0);
+    }
+    {
+        const uint64_t no = pack2(-t.o.y, -t.o.y), iv = pack2(t.inv.y, t.inv.y);
+        slab4(ny, no, iv, n1);
+        slab4(fy, no, iv, f1);
+    }
+    {
+        const uint64_t no = pack2(-t.o.z, -t.o.z), iv = pack2(t.inv.z, t.inv.z);
+        slab4(nz, no, iv, n2);
+        slab4(fz, no, iv, f2);
+    }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const float tnx = (n0[i] - t.o.x) * t.inv.x, tfx = (f0[i] - t.o.x) * t.inv.x;
-        const float tny = (n1[i] - t.o.y) * t.inv.y, tfy = (f1[i] - t.o.y) * t.inv.y;
-        const float tnz = (n2[i] - t.o.z) * t.inv.z, tfz = (f2[i] - t.o.z) * t.inv.z;
-        const float a = fmaxf(fmaxf(tnx, tny), fmaxf(tnz, t.tmin));
-        const float b = fminf(fminf(tfx, tfy), fminf(tfz, t.tmax));
-        key[i] = (a <= b && ref[i] != kEmpty) ? packKey(a, i) : kMissKey;
+        const float a = fmaxf(max3(n0[i], n1[i], n2[i]), t.tmin);
+        const float b = fminf(min3(f0[i], f1[i], f2[i]), t.tmax);
+        key[i] = a <= b ? packKey(a, i) : kMissKey;
     }
 }
 
-// Pops one entry: restores the world ray at a sentinel, tests an inner node and pushes its
-// hit children nearest-last, or makes a leaf pending. Returns an error bitmask. Without
-// ORDER (any-hit queries, whose answer does not depend on the visit order) the hit
+// Gives the lane reference `e` to work on: an inner node, or a leaf to hold.
+__device__ __forceinline__ void travTake(Trav& t, uint32_t e) {
+    const bool leaf = isLeaf(e);
+    t.leaf = leaf ? e : kEmpty;
+    t.cur = leaf ? kEmpty : e;
+}
+
+// Takes the next stack entry that is not beyond the nearest hit; a sentinel on the way
+// restores the world ray (Src::world). With an empty stack the lane holds nothing.
+template <bool CULL, typename Stack, typename Src>
+__device__ __forceinline__ void travPop(Trav& t, const Stack& st, const Src& src) {
+    t.cur = kEmpty;
+    t.leaf = kEmpty;
+    uint32_t cull = kMissKey;
+    if constexpr (CULL) cull = cullKey(t);
+    while (t.sp > 0) {
+        const auto e = st.get(--t.sp);
+        if (e.ref == kSentinel) {
+            const V3 od = t.d;
+            src.world(t.o, t.d, t.tmin);
+            if (!(od.x == t.d.x && od.y == t.d.y && od.z == t.d.z)) t.inv = v3(__frcp_rn(t.d.x), __frcp_rn(t.d.y), __frcp_rn(t.d.z));
+            t.fast = t.wfast;
+            t.curInst = -1;
+            if constexpr (CULL) cull = cullKey(t);
+            continue;
+        }
+        if constexpr (CULL) {
+            if (e.key > cull) continue;
+        }
+        travTake(t, e.ref);
+        return;
+    }
+}
+
+// Tests the lane's inner node: the nearest hit child is taken, the others are pushed
+// nearest last; without a hit the next stack entry is taken. Returns an error bitmask.
+// Without ORDER (any-hit queries, whose answer does not depend on the visit order) the hit
 // children are visited in slot order, which saves the sort.
-template <int BLOCK, bool COUNT, int SMEM, bool ORDER = true>
-__device__ __forceinline__ int travNodeStep(Trav& t, const SceneView& s, TStack<BLOCK, SMEM>& st, TraceCounters* cnt) {
-    uint32_t e;
-    if (t.next != kEmpty) {
-        e = t.next;
-        t.next = kEmpty;
-    } else {
-        e = st.get(--t.sp);
-    }
-    if (e == kSentinel) {
-        t.o = t.wo; t.d = t.wd;
-        t.inv = v3(__frcp_rn(t.wd.x), __frcp_rn(t.wd.y), __frcp_rn(t.wd.z));
-        t.fast = t.wfast;
-        t.tmin = t.wtmin;
-        t.curInst = -1;
-        return 0;
-    }
-    if (isLeaf(e)) {
-        t.leaf = e;
-        return 0;
-    }
-    const Node4* nd = s.nodes + e;
+template <bool COUNT, bool CULL, bool ORDER, typename Stack, typename Src>
+__device__ __forceinline__ int travNodeStep(Trav& t, const Node4* __restrict__ nodes, Stack& st, const Src& src, TraceCounters* cnt) {
+    const Node4* nd = nodes + t.cur;
     if (COUNT) cnt->nodes++;
     uint32_t key[4];
-    {
-        const uint4 ch = ldgu4(nd->child);
-        const uint32_t ref[4] = {ch.x, ch.y, ch.z, ch.w};
-        if (t.fast) nodeKeysFast(nd, t, ref, key);
-        else nodeKeysExact(nd, t, ref, key);
-    }
+    const uint4 ch = ldgu4(nd->child);   // with the boxes: a load after the sort would be another L1 latency
+    if (t.fast) nodeKeysFast(nd, t, key);
+    else nodeKeysExact(nd, t, key);
     if (!ORDER) {
+        const uint32_t ref[4] = {ch.x, ch.y, ch.z, ch.w};
         const int nhit = (key[0] != kMissKey) + (key[1] != kMissKey) + (key[2] != kMissKey) + (key[3] != kMissKey);
-        if (nhit == 0) return 0;
+        if (nhit == 0) {
+            travPop<CULL>(t, st, src);
+            return 0;
+        }
         if (t.sp + nhit - 1 > kPStackMax) return kTraceStackOverflow;
         uint32_t pending = kEmpty;
 #pragma unroll
         for (int i = 3; i >= 0; --i) {
             if (key[i] == kMissKey) continue;
-            if (pending != kEmpty) st.put(t.sp++, pending);
-            pending = __ldg(nd->child + i);
+            if (pending != kEmpty) st.put(t.sp++, pending, 0u);
+            pending = ref[i];
         }
-        t.next = pending;
+        travTake(t, pending);
         return 0;
     }
     // ascending sort network on the packed keys (unsigned min / max)
@@ -482,73 +563,64 @@ __device__ __forceinline__ int travNodeStep(Trav& t, const SceneView& s, TStack<
     }
     GND_CSWAP(0, 1) GND_CSWAP(2, 3) GND_CSWAP(0, 2) GND_CSWAP(1, 3) GND_CSWAP(1, 2)
 #undef GND_CSWAP
-    if (key[0] == kMissKey) return 0;
-    const int npush = (key[1] != kMissKey) + (key[2] != kMissKey) + (key[3] != kMissKey);
-    if (t.sp + npush > kPStackMax) return kTraceStackOverflow;
-    // farther children on the stack (farthest deepest), the nearest visited next
+    if (key[0] == kMissKey) {
+        travPop<CULL>(t, st, src);
+        return 0;
+    }
+    if (t.sp + 3 > kPStackMax && t.sp + (key[1] != kMissKey) + (key[2] != kMissKey) + (key[3] != kMissKey) > kPStackMax)
+        return kTraceStackOverflow;
+    // farther children on the stack (farthest deepest)
+    auto refOf = [&](uint32_t k) {
+        const uint32_t lo = (k & 1u) ? ch.y : ch.x, hi = (k & 1u) ? ch.w : ch.z;
+        return (k & 2u) ? hi : lo;
+    };
 #pragma unroll
     for (int i = 3; i >= 1; --i)
-        if (key[i] != kMissKey) st.put(t.sp++, __ldg(nd->child + (key[i] & 3u)));
-    t.next = __ldg(nd->child + (key[0] & 3u));
+        if (key[i] != kMissKey) st.put(t.sp++, refOf(key[i]), key[i]);
+    travTake(t, refOf(key[0]));
     return 0;
 }
 
-// Processes one primitive of the pending leaf. For ANY, a hit ends the ray (sp = 0).
-template <int BLOCK, bool ANY, bool COUNT, int SMEM, bool MOTION>
-__device__ __forceinline__ int travLeafStep(Trav& t, const SceneView& s, TStack<BLOCK, SMEM>& st, TraceCounters* cnt,
-                                            const uint8_t* nullMask) {
-    // the pending leaf's first primitive; the rest stays pending
+__device__ __forceinline__ void travStop(Trav& t) {
+    t.sp = 0;
+    t.cur = t.leaf = kEmpty;
+}
+
+// One instance of the pending top-level leaf; the rest of the leaf stays pending, or goes to
+// the stack when a mesh is entered. For ANY, a hit ends the ray.
+template <bool ANY, bool MOTION, typename Stack>
+__device__ __forceinline__ int travInstStep(Trav& t, const SceneView& s, Stack& st, const uint8_t* nullMask, float time) {
     const uint32_t first = leafFirst(t.leaf), count = leafCount(t.leaf);
     t.leaf = count > 1u ? makeLeaf(first + 1u, count - 1u) : kEmpty;
-    if (t.curInst >= 0) {
-        float tt, u, v;
-        uint32_t prim;
-        if (COUNT) cnt->tris++;
-        if (triTest(s.tris + first, t.o, t.d, t.tmin, t.tmax, tt, u, v, prim)) {
-            t.tmax = tt;
-            t.bestT = tt;
-            t.hit.u = u; t.hit.v = v;
-            t.hit.inst = t.curInst;
-            t.hit.slot = first;
-            if (ANY) { t.sp = 0; t.leaf = kEmpty; t.next = kEmpty; }
-        }
-        return 0;
-    }
     uint32_t id = __ldg(s.tlasList + first);
     if (nullMask && nullMask[id]) return 0;
     const InstTrav* it = s.instT + id;
     float4 r0 = ldg4(&it->w2o.r[0][0]), r1 = ldg4(&it->w2o.r[1][0]), r2 = ldg4(&it->w2o.r[2][0]);
     float4 meta = ldg4(&it->kind);
     uint32_t kind = __float_as_uint(meta.x);
-    if (MOTION && (kind & kInstAnimated)) animatedW2ORows(s, id, t.time, r0, r1, r2);
+    if (MOTION && (kind & kInstAnimated)) animatedW2ORows(s, id, time, r0, r1, r2);
     kind &= ~kInstAnimated;
     V3 lo, ld;
-    lo.x = (r0.x * t.wo.x + r0.y * t.wo.y) + (r0.z * t.wo.z + r0.w);
-    lo.y = (r1.x * t.wo.x + r1.y * t.wo.y) + (r1.z * t.wo.z + r1.w);
-    lo.z = (r2.x * t.wo.x + r2.y * t.wo.y) + (r2.z * t.wo.z + r2.w);
-    ld.x = (r0.x * t.wd.x + r0.y * t.wd.y) + (r0.z * t.wd.z + r0.w * 0.0f);
-    ld.y = (r1.x * t.wd.x + r1.y * t.wd.y) + (r1.z * t.wd.z + r1.w * 0.0f);
-    ld.z = (r2.x * t.wd.x + r2.y * t.wd.y) + (r2.z * t.wd.z + r2.w * 0.0f);
+    lo.x = (r0.x * t.o.x + r0.y * t.o.y) + (r0.z * t.o.z + r0.w);
+    lo.y = (r1.x * t.o.x + r1.y * t.o.y) + (r1.z * t.o.z + r1.w);
+    lo.z = (r2.x * t.o.x + r2.y * t.o.y) + (r2.z * t.o.z + r2.w);
+    ld.x = (r0.x * t.d.x + r0.y * t.d.y) + (r0.z * t.d.z + r0.w * 0.0f);
+    ld.y = (r1.x * t.d.x + r1.y * t.d.y) + (r1.z * t.d.z + r1.w * 0.0f);
+    ld.z = (r2.x * t.d.x + r2.y * t.d.y) + (r2.z * t.d.z + r2.w * 0.0f);
     if (kind == kShapeMesh) {
         uint32_t root = __float_as_uint(meta.y);
         if (root == kEmpty) return 0;
-        if (t.next != kEmpty) {
-            // an entry found by speculative traversal before this leaf: keep it for later
-            if (t.sp >= kPStackMax) return kTraceStackOverflow;
-            st.put(t.sp++, t.next);
-            t.next = kEmpty;
-        }
+        if (t.sp + 1 + (t.leaf != kEmpty) > kPStackMax) return kTraceStackOverflow;
         if (t.leaf != kEmpty) {
             // the rest of this leaf comes back after the bottom-level tree
-            if (t.sp >= kPStackMax) return kTraceStackOverflow;
-            st.put(t.sp++, t.leaf);
+            st.put(t.sp++, t.leaf, 0u);
             t.leaf = kEmpty;
         }
-        if (t.sp + 1 > kPStackMax) return kTraceStackOverflow;
-        st.put(t.sp++, kSentinel);
-        t.next = root;   // the bottom-level root is visited next
+        st.put(t.sp++, kSentinel, 0u);
+        t.cur = root;
+        // a translation keeps the direction, and with it the three reciprocals
+        if (!(ld.x == t.d.x && ld.y == t.d.y && ld.z == t.d.z)) t.inv = v3(__frcp_rn(ld.x), __frcp_rn(ld.y), __frcp_rn(ld.z));
         t.o = lo; t.d = ld;
-        t.inv = v3(__frcp_rn(ld.x), __frcp_rn(ld.y), __frcp_rn(ld.z));
         t.fast = t.wfast && slabFinite(s, lo, t.inv);
         t.tmin = kEpsilon;
         t.curInst = (int)id;
@@ -558,21 +630,86 @@ __device__ __forceinline__ int travLeafStep(Trav& t, const SceneView& s, TStack<
     bool h;
     if (kind == kShapeSphere) h = sphereTest(meta.z, lo, ld, kEpsilon, t.tmax, th);
     else h = cubeTest(v3(meta.z, meta.w, __ldg(&s.instS[id].ext[2])), lo, ld, kEpsilon, t.tmax, th);
-    if (h && th < t.bestT) {
+    // bvh.cpp:39: the nearest distance starts at FLT_MAX
+    if (h && th < (t.inst >= 0 ? t.tmax : 3.402823466e38f)) {
         t.tmax = th;
-        t.bestT = th;
-        t.hit.u = 0.f; t.hit.v = 0.f;
-        t.hit.inst = (int)id;
-        t.hit.slot = 0xFFFFFFFFu;
-        if (ANY) { t.sp = 0; t.leaf = kEmpty; t.next = kEmpty; }
+        t.u = t.v = 0.0f;
+        t.inst = (int)id;
+        t.slot = 0xFFFFFFFFu;
+        if (ANY) travStop(t);
     }
     return 0;
 }
 
-// The hit a finished query reports: every accepted hit sets bestT to its distance.
+// Tests triangles of the lanes' pending bottom-level leaves: up to four of each lane's leaf,
+// up to 32 in all, one per lane of the warp (all lanes call it; `mine`: this lane holds such
+// a leaf). The owner's ray comes by shuffle; the owner then takes the nearest hit of its
+// triangles, the first of equal ones as a loop over them would. Lanes whose triangles do not
+// fit keep their leaf for the next pass. `map`: this warp's 32 words of shared memory.
+// On random rays a leaf holds 1.8 triangles: one pass of 21 busy lanes takes the place of 3.5
+// steps with 6.
+template <bool ANY, bool COUNT>
+__device__ __forceinline__ void travTriPass(Trav& t, const SceneView* sv, bool mine, uint32_t* map, TraceCounters* cnt) {
+    const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    const uint32_t first = leafFirst(t.leaf), count = mine ? leafCount(t.leaf) : 0u;
+    const uint32_t take = min(count, 4u);
+    const uint32_t m = __ballot_sync(0xffffffffu, mine);
+    const uint32_t c0 = __ballot_sync(0xffffffffu, mine && ((take - 1u) & 1u)), c1 = __ballot_sync(0xffffffffu, mine && ((take - 1u) & 2u));
+    const uint32_t at = (uint32_t)__popc(m & below) + (uint32_t)__popc(c0 & below) + 2u * (uint32_t)__popc(c1 & below);
+    const bool fits = mine && at + take <= 32u;
+    // owner of pair p: the lane whose range starts at the last start at or below p
+    const uint32_t starts = __reduce_or_sync(0xffffffffu, fits ? 1u << at : 0u);
+    const uint32_t total = __reduce_max_sync(0xffffffffu, fits ? at + take : 0u);
+    if (fits) map[at] = lane;
+    __syncwarp();
+    const bool busy = lane < total;
+    const int start = 31 - __clz((int)(starts & (below | (1u << lane))));
+    const uint32_t owner = busy ? map[start] : lane;
+    __syncwarp();
+    TRay r;
+    r.o.x = __shfl_sync(0xffffffffu, t.o.x, owner); r.o.y = __shfl_sync(0xffffffffu, t.o.y, owner);
+    r.o.z = __shfl_sync(0xffffffffu, t.o.z, owner);
+    r.d.x = __shfl_sync(0xffffffffu, t.d.x, owner); r.d.y = __shfl_sync(0xffffffffu, t.d.y, owner);
+    r.d.z = __shfl_sync(0xffffffffu, t.d.z, owner);
+    r.tmin = __shfl_sync(0xffffffffu, t.tmin, owner);
+    r.tmax = __shfl_sync(0xffffffffu, t.tmax, owner);
+    const Tri* tris = reinterpret_cast<const Tri*>(
+        __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(mine ? sv->tris + first : nullptr), owner));
+    float th = INFINITY, u = 0.0f, v = 0.0f;
+    if (busy) {
+        float tt;
+        uint32_t prim;
+        if (triTest(tris + (lane - (uint32_t)start), r.o, r.d, r.tmin, r.tmax, tt, u, v, prim)) th = tt;
+    }
+    uint32_t best = 32u;
+    if (__any_sync(0xffffffffu, th < INFINITY)) {
+#pragma unroll
+        for (uint32_t k = 0; k < 4u; ++k) {
+            const float c = __shfl_sync(0xffffffffu, th, (at + k) & 31u);
+            if (fits && k < take && c < t.tmax) { t.tmax = c; best = k; }
+        }
+        const uint32_t from = (at + best) & 31u;
+        const float bu = __shfl_sync(0xffffffffu, u, from), bv = __shfl_sync(0xffffffffu, v, from);
+        if (best < 4u) {
+            t.u = bu; t.v = bv;
+            t.inst = t.curInst;
+            t.slot = first + best;
+        }
+    }
+    if (fits) {
+        if (COUNT) cnt->tris += take;
+        t.leaf = count > take ? makeLeaf(first + take, count - take) : kEmpty;
+        if (ANY && best < 4u) travStop(t);
+    }
+}
+
+// The hit a finished query reports.
 __device__ __forceinline__ THit travHit(const Trav& t) {
-    THit h = t.hit;
-    h.t = t.hit.inst >= 0 ? t.bestT : INFINITY;
+    THit h;
+    h.t = t.inst >= 0 ? t.tmax : INFINITY;
+    h.u = t.u; h.v = t.v;
+    h.inst = t.inst;
+    h.slot = t.slot;
     return h;
 }
 
@@ -593,6 +730,7 @@ __device__ __forceinline__ uint32_t warpFetch(uint32_t* counter, bool want) {
 // is a multiple of 32 and no lane exits early). Src provides:
 //   uint32_t count()                      number of rays
 //   bool load(uint32_t i, TRay&, const SceneView*&, const uint8_t*& nullMask)
+//   void world(V3& o, V3& d, float& tmin) const   the ray in flight again (leaving a mesh)
 //   void store(uint32_t i, const THit&, const SceneView&)   (the query's scene)
 // SLOT_ORDER_ANY: any-hit queries visit hit children in slot order instead of nearest
 // first (faster for the bounded shadow segments of the path tracer; rays to infinity find
@@ -600,85 +738,106 @@ __device__ __forceinline__ uint32_t warpFetch(uint32_t* counter, bool want) {
 // leafBatch (1..32): the node phase ends as soon as that many lanes hold a leaf (32: when
 // no lane can take another node step); lanes still traversing keep their state and go on
 // in the next round. Only the interleaving of the lanes' steps changes.
-template <int BLOCK, bool ANY, bool COUNT, int SMEM = kSmemStack, bool SPEC = false, bool MOTION = false,
-          bool SLOT_ORDER_ANY = false, typename Src>
-__device__ __forceinline__ int persistentTrace(Src& src, uint32_t* fetchCounter, uint32_t* smemStack, TraceCounters* cnt,
-                                               uint32_t leafBatch = 32) {
-    TStack<BLOCK, SMEM> st;
+// `map`: 32 words of shared memory per warp.
+// Measured (one B200; 4.2M random rays on 2^20 triangles / 32 passes of the 1024^2 sphere grid):
+// full node phases, refill of any idle lane 2.30 ms / 101.6 ms, one child per step, triangle by
+// triangle; this loop 1.77 / 88.5. Its parts: kPassLanes 32, 24, 16, 12: - / 98.9, 95.3, 94.1,
+// 95.9; kRefill 1, 4, 8, 12: 1.94, 1.90, 1.88, 1.94 / -, 93.0, 91.5, -; child references loaded
+// with the boxes instead of after the sort -4% / -0.7%; reciprocals kept across a translation
+// -1.5% / -2%. Two steps per vote, 7 or 6 blocks per SM: no gain on the small scenes.
+constexpr int kPassLanes = 16;
+constexpr int kRefill = 8;
+template <int BLOCK, bool ANY, bool COUNT, int SMEM = kSmemStack, bool MOTION = false, bool SLOT_ORDER_ANY = false, typename Src>
+__device__ __forceinline__ int persistentTrace(Src& src, uint32_t* fetchCounter, TEntry<!ANY>* smemStack, uint32_t* smemMap,
+                                               TraceCounters* cnt, uint32_t leafBatch = 32) {
+    constexpr bool kCull = !ANY && !COUNT;   // the counting variants count the plain traversal's visits
+    // a leaf pass takes 32 triangles: waiting for more than kPassLanes lanes gains nothing
+    if (!COUNT) leafBatch = min(leafBatch, (uint32_t)kPassLanes);
+    TStack<BLOCK, SMEM, !ANY> st;
     st.smem = smemStack + threadIdx.x;
+    uint32_t* map = smemMap + (threadIdx.x & ~31u);
     Trav t;
+    travStop(t);
     const SceneView* sv = nullptr;
+    const Node4* nodes = nullptr;
     const uint8_t* nm = nullptr;
+    float time = 0.0f;
     bool active = false;
     bool drained = false;   // warp-uniform: the counter has passed n
     uint32_t idx = 0;
     int err = 0;
     const uint32_t n = src.count();
     uint32_t iter = 0;
+    // Fewer rays than lanes: spread over all warps, since a warp's steps grow with the number
+    // of its lanes that diverge. (1000 rays: a warp each.)
+    const uint32_t warps = gridDim.x * (BLOCK / 32);
+    // At least one lane takes rays, to see that there are none left.
+    const bool takes = (threadIdx.x & 31u) < (n < warps * 32u ? max((n + warps - 1u) / warps, 1u) : 32u);
     for (;;) {
-        bool idle = !active && !drained;
-        uint32_t got = warpFetch(fetchCounter, idle);
-        if (__any_sync(0xffffffffu, idle && got >= n)) drained = true;
-        if (idle && got < n) {
-            idx = got;
-            TRay r;
-            // a source may decline an item (it belongs to another kernel of the launch)
-            if (src.load(idx, r, sv, nm)) {
-                travInit(t, *sv, r);
-                // kEmpty for a scene without primitives; the counting variants report what
-                // the traversal visits, a NaN ray's too
-                t.next = !COUNT && missesAll(*sv, r) ? kEmpty : sv->tlasRoot;
-                active = true;
-                iter = 0;
+        // new rays when kRefill lanes are out of work (or all): setting up a ray costs about
+        // a node step, whatever the number of lanes doing it
+        const uint32_t busy = __ballot_sync(0xffffffffu, active);
+        if (!drained && __popc(busy) <= 32 - kRefill) {
+            const bool idle = !active && takes;
+            const uint32_t got = warpFetch(fetchCounter, idle);
+            if (__any_sync(0xffffffffu, idle && got >= n)) drained = true;
+            if (idle && got < n) {
+                idx = got;
+                TRay r;
+                // a source may decline an item (it belongs to another kernel of the launch)
+                if (src.load(idx, r, sv, nm)) {
+                    travInit(t, *sv, r);
+                    // the counting variants report what the traversal visits, a NaN ray's too
+                    if (!COUNT && !t.fast && missesAll(*sv, r)) t.cur = kEmpty;
+                    nodes = sv->nodes;
+                    if (MOTION) time = r.time;
+                    active = true;
+                    iter = 0;
+                }
             }
         }
-        if (!__any_sync(0xffffffffu, active)) break;
-        // node phase. Without SPEC a lane steps until it holds a leaf. With SPEC every lane
-        // steps until it is blocked: a lane that holds a leaf keeps traversing ahead while
-        // its next entry is an inner node of the same tree, and stops at the next leaf,
-        // sentinel or an empty stack (more lanes busy per step, at the price of visits a
-        // shorter tMax would have culled). Either way whether a lane steps depends only on
+        if (!__any_sync(0xffffffffu, active)) {
+            if (drained) break;
+            continue;
+        }
+        // node phase: a lane steps until it holds a leaf. Whether it steps depends only on
         // its own state, so each ray's sequence of visits, and its result, is the same
         // whatever the other rays of the warp do.
         for (;;) {
-            const bool work = t.next != kEmpty || t.sp > 0;
-            bool want = active && work;
-            if (want && t.leaf != kEmpty) {
-                if (!SPEC) {
-                    want = false;
-                } else {
-                    const uint32_t peek = t.next != kEmpty ? t.next : st.get(t.sp - 1);
-                    want = peek != kSentinel && !isLeaf(peek);
-                }
-            }
-            if (!__any_sync(0xffffffffu, want)) break;
-            if (leafBatch < 32u && (uint32_t)__popc(__ballot_sync(0xffffffffu, active && t.leaf != kEmpty)) >= leafBatch)
-                break;
+            const bool want = t.cur != kEmpty;
+            const uint32_t wants = __ballot_sync(0xffffffffu, want);
+            if (!wants) break;
+            if ((uint32_t)__popc(__ballot_sync(0xffffffffu, t.leaf != kEmpty)) >= leafBatch) break;
             if (COUNT && (threadIdx.x & 31) == 0) cnt->nodeWarpSteps++;
             if (want) {
-                int e = travNodeStep<BLOCK, COUNT, SMEM, !(ANY && SLOT_ORDER_ANY)>(t, *sv, st, cnt);
+                const int e = travNodeStep<COUNT, kCull, !(ANY && SLOT_ORDER_ANY)>(t, nodes, st, src, cnt);
                 if (e || ++iter > kMaxIterations) {
                     err |= e ? e : (int)kTraceIterLimit;
-                    t.sp = 0; t.leaf = kEmpty; t.next = kEmpty;
+                    travStop(t);
                 }
             }
         }
-        // leaf phase
-        for (;;) {
-            bool want = active && t.leaf != kEmpty;
-            if (!__any_sync(0xffffffffu, want)) break;
-            if (COUNT) {
-                if ((threadIdx.x & 31) == 0) cnt->leafWarpSteps++;
-                if (want) cnt->leafSteps++;
-            }
-            if (want) {
-                int e = travLeafStep<BLOCK, ANY, COUNT, SMEM, MOTION>(t, *sv, st, cnt, nm);
-                if (e) { err |= e; t.sp = 0; t.leaf = kEmpty; t.next = kEmpty; }
+        // leaf pass
+        const bool held = t.leaf != kEmpty;
+        const bool tri = held && t.curInst >= 0;
+        if (COUNT && __any_sync(0xffffffffu, held)) {
+            if ((threadIdx.x & 31) == 0) cnt->leafWarpSteps++;
+            if (held) cnt->leafSteps++;
+        }
+        if (__any_sync(0xffffffffu, tri)) travTriPass<ANY, COUNT>(t, sv, tri, map, cnt);
+        if (held && !tri) {
+            const int e = travInstStep<ANY, MOTION>(t, *sv, st, nm, time);
+            if (e) {
+                err |= e;
+                travStop(t);
             }
         }
-        if (active && t.sp == 0 && t.leaf == kEmpty && t.next == kEmpty) {
-            src.store(idx, travHit(t), *sv);
-            active = false;
+        if (t.leaf == kEmpty && t.cur == kEmpty) {
+            if (t.sp > 0) travPop<kCull>(t, st, src);
+            if (active && t.sp == 0 && t.leaf == kEmpty && t.cur == kEmpty) {
+                src.store(idx, travHit(t), *sv);
+                active = false;
+            }
         }
     }
     return err;

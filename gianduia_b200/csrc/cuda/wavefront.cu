@@ -29,6 +29,7 @@
 namespace gnd {
 
 constexpr int kBlock = 128;
+constexpr int kTravBlocks = 8;             // blocks per SM the traversal kernels are compiled to fit
 constexpr float kFixScale = 16777216.0f;   // 2^24
 constexpr float kFixMax = 1e11f;           // per-sample clamp before the fixed-point conversion
 // Shade classes: integrator (0 path, 1 volpath) x class. Classes 0..3 follow the
@@ -846,19 +847,27 @@ struct ExtendSrc {
         hr.pad[1] = hr.pad[2] = 0;
         p->hits[slot] = hr;
     }
+    __device__ void world(V3& o, V3& d, float& tmin) const {
+        const PathState* ps = p->paths + slot;
+        const float4 a = *reinterpret_cast<const float4*>(&ps->ox);
+        const float4 b = *reinterpret_cast<const float4*>(&ps->dx);
+        o = v3(a.x, a.y, a.z);
+        d = v3(b.x, b.y, b.z);
+        tmin = kEpsilon;
+    }
 };
 
-// MOTION: the scene has animated instances (rays carry their shutter time)
-// MINB: the blocks per SM the kernel is compiled to fit (8: 64 registers; 9 and 10 trade
-// registers, with some spilled, for more resident warps; gnd_tune trav_blocks)
-template <bool COUNT, int SMEM, bool SPEC, bool MOTION = false, int MINB = 8>
-__global__ void __launch_bounds__(kBlock, MINB) kExtend(KParams p) {
-    __shared__ uint32_t stack[SMEM * kBlock];
+// MOTION: the scene has animated instances (rays carry their shutter time). SMEM: stack
+// entries in shared memory.
+template <bool COUNT, int SMEM, bool MOTION>
+__global__ void __launch_bounds__(kBlock, kTravBlocks) kExtend(KParams p) {
+    __shared__ TEntry<true> stack[SMEM * kBlock];
+    __shared__ uint32_t map[kBlock];
     const uint32_t n = p.cnt[kQIn];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&p.totals[0], (unsigned long long)n);
     TraceCounters cnt{0, 0, 0, 0, 0};
     ExtendSrc src{&p, n, 0};
-    int err = persistentTrace<kBlock, false, COUNT, SMEM, SPEC, MOTION>(src, p.cnt + kQFetchA, stack, &cnt, p.leafBatch);
+    int err = persistentTrace<kBlock, false, COUNT, SMEM, MOTION>(src, p.cnt + kQFetchA, stack, map, &cnt, p.leafBatch);
     if (COUNT) {
         unsigned long long nn = cnt.nodes, nt = cnt.tris, nw = cnt.nodeWarpSteps, ls = cnt.leafSteps, lw = cnt.leafWarpSteps;
         for (int o = 16; o > 0; o >>= 1) {
@@ -1236,7 +1245,15 @@ struct ShadowSrc {
         nmOut = nullptr;
         return true;
     }
-    __device__ void store(uint32_t i, const THit& h, const SceneView&) {
+    __device__ void world(V3& o, V3& d, float& tmin) const {
+        const ShadowRec* sr = p->shadow + rec;
+        const float4 a = *reinterpret_cast<const float4*>(&sr->ox);
+        const float4 b = *reinterpret_cast<const float4*>(&sr->dx);
+        o = v3(a.x, a.y, a.z);
+        d = v3(b.x, b.y, b.z);
+        tmin = kEpsilon;
+    }
+    __device__ void store(uint32_t, const THit& h, const SceneView&) {
         const ShadowRec* sr = p->shadow + rec;
         const uint32_t slot = sr->slot;
         PathState* ps = p->paths + slot;
@@ -1250,20 +1267,20 @@ struct ShadowSrc {
     }
 };
 
-template <bool ANY, int SMEM, bool SPEC, bool MOTION = false, int MINB = 8>
-__global__ void __launch_bounds__(kBlock, MINB) kShadowPath(KParams p, bool mixed) {
-    __shared__ uint32_t stack[SMEM * kBlock];
+template <bool ANY, int SMEM, bool MOTION>
+__global__ void __launch_bounds__(kBlock, kTravBlocks) kShadowPath(KParams p, bool mixed) {
+    __shared__ TEntry<!ANY> stack[SMEM * kBlock];
+    __shared__ uint32_t map[kBlock];
     const uint32_t n = p.cnt[kQShadow];
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&p.totals[1], (unsigned long long)n);
     ShadowSrc<ANY> src{&p, n, mixed, 0};
-    int err = persistentTrace<kBlock, ANY, false, SMEM, SPEC, MOTION, true>(src, p.cnt + kQFetchB, stack, nullptr,
-                                                                            p.shadowLeafBatch);
+    int err = persistentTrace<kBlock, ANY, false, SMEM, MOTION, true>(src, p.cnt + kQFetchB, stack, map, nullptr, p.shadowLeafBatch);
     if (err) atomicOr(p.errWord, (uint32_t)err);
 }
 
 // Shadow queries of `volpath`: evaluateTr (volPath.cpp:261-291), a loop of closest hits
 // through null-BSDF boundaries multiplying the transmittance of each medium segment.
-template <bool VOL, bool MOTION = false>
+template <bool MOTION>
 __global__ void __launch_bounds__(kBlock) kShadow(KParams p, bool mixed) {
     __shared__ uint32_t stack[kStackSize * kBlock];
     uint32_t* stk = stack + threadIdx.x;
@@ -1285,23 +1302,14 @@ __global__ void __launch_bounds__(kBlock) kShadow(KParams p, bool mixed) {
         r.time = __uint_as_float(sr.pad);
         V3 c = v3(sr.cr, sr.cg, sr.cb);
         bool clear;
-        if (!VOL) {
-            THit h;
-            if (j.hasNull) {
-                err |= traceRay<kBlock, false, false, false, MOTION>(s, r, h, stk, nullptr, nullptr);
-                clear = h.inst < 0 || j.nullMask[h.inst];
-            } else {
-                err |= traceRay<kBlock, true, false, false, MOTION>(s, r, h, stk, nullptr, nullptr);
-                clear = h.inst < 0;
-            }
-        } else {
+        {
             V3 Tr = v3s(1.0f);
             int medium = sr.medium;
             V3 lightP = v3(sr.lx, sr.ly, sr.lz);
             clear = true;
             for (int seg = 0; seg < 256; ++seg) {
                 THit h;
-                err |= traceRay<kBlock, false, false, false, MOTION>(s, r, h, stk, nullptr, nullptr);
+                err |= traceRay<kBlock, MOTION>(s, r, h, stk);
                 bool hit = h.inst >= 0;
                 if (medium >= 0) {
                     float segT = hit ? h.t : r.tmax;
@@ -1981,62 +1989,32 @@ void Wavefront::drop(int j) {
     syncActive();
 }
 
-// The plain traversal kernels compiled for MINB blocks per SM.
-template <int SMEM, int MINB>
-static void launchWide(const KParams& kp, int mix, bool hasNull, int travGrid, cudaStream_t st, cudaEvent_t ea,
-                       cudaEvent_t eb, int stage) {
+// The extend kernel (stage 0, between events ea and eb when given) or the path integrator's
+// shadow kernel (stage 1). count: the instrumented extend kernel (static scenes).
+template <int SMEM, bool MOTION>
+static void launchTraversal(const KParams& kp, int mix, bool hasNull, bool count, int travGrid, cudaStream_t st,
+                            cudaEvent_t ea, cudaEvent_t eb, int stage) {
     if (stage == 0) {
         if (ea) GND_CUDA(cudaEventRecord(ea, st));
-        kExtend<false, SMEM, false, false, MINB><<<travGrid, kBlock, 0, st>>>(kp);
+        if (count && !MOTION) kExtend<true, SMEM, false><<<travGrid, kBlock, 0, st>>>(kp);
+        else kExtend<false, SMEM, MOTION><<<travGrid, kBlock, 0, st>>>(kp);
         if (eb) GND_CUDA(cudaEventRecord(eb, st));
     } else if (mix & 1) {
-        if (hasNull) kShadowPath<false, SMEM, false, false, MINB><<<travGrid, kBlock, 0, st>>>(kp, mix == 3);
-        else kShadowPath<true, SMEM, false, false, MINB><<<travGrid, kBlock, 0, st>>>(kp, mix == 3);
+        if (hasNull) kShadowPath<false, SMEM, MOTION><<<travGrid, kBlock, 0, st>>>(kp, mix == 3);
+        else kShadowPath<true, SMEM, MOTION><<<travGrid, kBlock, 0, st>>>(kp, mix == 3);
     }
 }
 
-// The traversal kernels for one shared-stack size and speculation setting; bps: blocks
-// per SM (the grid is bps per SM; 9 and 10 select the kernels compiled for them, for
-// static scenes without speculation or visit counting).
-template <int SMEM, bool SPEC>
-static void launchTraversal(const KParams& kp, int mix, bool hasNull, bool count, int travGrid, cudaStream_t st,
-                            cudaEvent_t ea, cudaEvent_t eb, int stage, bool motion, int bps) {
-    if (!motion && !count && !SPEC && bps > 8) {
-        if (bps == 9) launchWide<SMEM, 9>(kp, mix, hasNull, travGrid, st, ea, eb, stage);
-        else launchWide<SMEM, 10>(kp, mix, hasNull, travGrid, st, ea, eb, stage);
-        return;
+void Wavefront::traversal(const KParams& kp, int mix, bool hasNull, bool count, cudaStream_t st, cudaEvent_t ea, cudaEvent_t eb,
+                          int stage) {
+    const int grid = ctx_->numSMs * std::min(std::max(tune_.travBlocks, 1), kTravBlocks);
+    if (tune_.smem == 16) {
+        if (motion_) launchTraversal<8, true>(kp, mix, hasNull, count, grid, st, ea, eb, stage);
+        else launchTraversal<8, false>(kp, mix, hasNull, count, grid, st, ea, eb, stage);
+    } else {
+        if (motion_) launchTraversal<16, true>(kp, mix, hasNull, count, grid, st, ea, eb, stage);
+        else launchTraversal<16, false>(kp, mix, hasNull, count, grid, st, ea, eb, stage);
     }
-    if (bps > 8) travGrid = travGrid / bps * 8;   // the 64-register kernels fit 8 blocks per SM
-    if (motion) {
-        // animated instances: the MOTION kernels (no speculation, no visit counters)
-        if (stage == 0) {
-            if (ea) GND_CUDA(cudaEventRecord(ea, st));
-            kExtend<false, SMEM, false, true><<<travGrid, kBlock, 0, st>>>(kp);
-            if (eb) GND_CUDA(cudaEventRecord(eb, st));
-        } else if (mix & 1) {
-            if (hasNull) kShadowPath<false, SMEM, false, true><<<travGrid, kBlock, 0, st>>>(kp, mix == 3);
-            else kShadowPath<true, SMEM, false, true><<<travGrid, kBlock, 0, st>>>(kp, mix == 3);
-        }
-        return;
-    }
-    if (stage == 0) {
-        if (ea) GND_CUDA(cudaEventRecord(ea, st));
-        // the instrumented variant counts the visits of plain nearest-first order: the
-        // algorithmic work of a ray, independent of speculation
-        if (count) kExtend<true, SMEM, false><<<travGrid, kBlock, 0, st>>>(kp);
-        else kExtend<false, SMEM, SPEC><<<travGrid, kBlock, 0, st>>>(kp);
-        if (eb) GND_CUDA(cudaEventRecord(eb, st));
-    } else if (mix & 1) {
-        if (hasNull) kShadowPath<false, SMEM, SPEC><<<travGrid, kBlock, 0, st>>>(kp, mix == 3);
-        else kShadowPath<true, SMEM, SPEC><<<travGrid, kBlock, 0, st>>>(kp, mix == 3);
-    }
-}
-
-template <int SMEM>
-static void launchTraversal(const KParams& kp, int mix, bool hasNull, bool count, int travGrid, cudaStream_t st,
-                            cudaEvent_t ea, cudaEvent_t eb, int stage, bool spec, bool motion, int bps) {
-    if (spec) launchTraversal<SMEM, true>(kp, mix, hasNull, count, travGrid, st, ea, eb, stage, motion, bps);
-    else launchTraversal<SMEM, false>(kp, mix, hasNull, count, travGrid, st, ea, eb, stage, motion, bps);
 }
 
 void Wavefront::setTune(const Tune& t) {
@@ -2048,8 +2026,6 @@ void Wavefront::setTune(const Tune& t) {
 
 void Wavefront::enqueueIteration(KParams kp, int par, int mix, bool hasNull, int profile, cudaStream_t st) {
     const int grid = ctx_->numSMs * 8;
-    const int bps = std::min(std::max(tune_.travBlocks, 1), 10);
-    const int travGrid = ctx_->numSMs * bps;
     const bool sort = tune_.sort != 0 || mix == 3;   // an unsorted launch serves one integrator
     uint32_t* lists[2] = {listA_.as<uint32_t>(), listB_.as<uint32_t>()};
     uint32_t* frees[2] = {freeA_.as<uint32_t>(), freeB_.as<uint32_t>()};
@@ -2074,8 +2050,7 @@ void Wavefront::enqueueIteration(KParams kp, int par, int mix, bool hasNull, int
         evs_.push_back(eb);
     }
     const bool count = (profile & 2) != 0;
-    if (tune_.smem == 16) launchTraversal<16>(kp, mix, hasNull, count, travGrid, st, ea, eb, 0, tune_.specExtend != 0, motion_, bps);
-    else launchTraversal<32>(kp, mix, hasNull, count, travGrid, st, ea, eb, 0, tune_.specExtend != 0, motion_, bps);
+    traversal(kp, mix, hasNull, count, st, ea, eb, 0);
     if (sort) {
         uint32_t* cls = classes_.as<uint32_t>();
         kClassify<<<ctx_->numSMs * 4, kAggBlock, 0, st>>>(kp, cls);   // latency-bound: a full SM of warps
@@ -2103,11 +2078,10 @@ void Wavefront::enqueueIteration(KParams kp, int par, int mix, bool hasNull, int
         kRayClear<<<64, 1024, 0, st>>>(kp.rayBins);
         kp.shadowOrder = kp.raySorted;
     }
-    if (tune_.smem == 16) launchTraversal<16>(kp, mix, hasNull, false, travGrid, st, nullptr, nullptr, 1, tune_.specShadow != 0, motion_, bps);
-    else launchTraversal<32>(kp, mix, hasNull, false, travGrid, st, nullptr, nullptr, 1, tune_.specShadow != 0, motion_, bps);
+    traversal(kp, mix, hasNull, false, st, nullptr, nullptr, 1);
     if (mix & 2) {
-        if (motion_) kShadow<true, true><<<grid, kBlock, 0, st>>>(kp, mix == 3);
-        else kShadow<true><<<grid, kBlock, 0, st>>>(kp, mix == 3);
+        if (motion_) kShadow<true><<<grid, kBlock, 0, st>>>(kp, mix == 3);
+        else kShadow<false><<<grid, kBlock, 0, st>>>(kp, mix == 3);
     }
     // 12 blocks per SM: its register limit
     if (ext_) kRetire<true><<<ctx_->numSMs * 3, kAggBlock, 0, st>>>(kp);
@@ -2534,9 +2508,9 @@ gnd_status gnd_gpu_autotune(gnd_gpu_ctx* ctxh, gnd_scene_id id, int32_t spp, int
             std::vector<int> values;
         };
         const std::vector<Knob> knobs = {
-            {&Tune::travBlocks, {8, 9, 10, 6, 4}}, {&Tune::smem, {32, 16}},          {&Tune::sort, {1, 0}},
+            {&Tune::travBlocks, {8, 6, 4}}, {&Tune::smem, {32, 16}},          {&Tune::sort, {1, 0}},
             {&Tune::poolLog2, {22, 21, 23, 24, 20}}, {&Tune::roundIters, {8, 16, 4}}, {&Tune::graphs, {1, 0}},
-            {&Tune::sampleFilm, {1, 0}}, {&Tune::specExtend, {1, 0}}, {&Tune::specShadow, {1, 0}},
+            {&Tune::sampleFilm, {1, 0}},
             {&Tune::raySort, {1, 3, 0}}, {&Tune::leafBatch, {16, 8, 24, 32}}, {&Tune::shadowLeafBatch, {16, 8, 24, 32}},
         };
         for (int sweep = 0; sweep < 2; ++sweep) {

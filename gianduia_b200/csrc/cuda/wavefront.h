@@ -177,6 +177,7 @@ private:
     void syncActive();
     // One wavefront iteration on the stream for the lists of parity `par`.
     void enqueueIteration(KParams kp, int par, int mix, bool hasNull, int profile, cudaStream_t st);
+    void traversal(const KParams& kp, int mix, bool hasNull, bool count, cudaStream_t st, cudaEvent_t ea, cudaEvent_t eb, int stage);
     // Executable graph of two iterations (parity restored) for these settings, captured on
     // first use; the per-iteration state it needs (queue counters, iteration number) is
     // in device memory, so one capture serves every later replay.

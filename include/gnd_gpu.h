@@ -398,20 +398,19 @@ gnd_status gnd_gpu_counters(gnd_gpu_ctx* ctx, gnd_counters* out, int32_t reset);
 typedef struct gnd_tune {
     int32_t pool_log2;        /* path slots of a batched render: 2^pool_log2 (16..26) */
     int32_t round_iters;      /* wavefront iterations per host round, batched (2..64, even) */
-    int32_t trav_blocks;      /* persistent traversal blocks of 128 threads per SM (1..10; 9
-                                 and 10 run the plain closest-hit and shadow kernels
-                                 compiled to fit them, with fewer registers per thread) */
+    int32_t trav_blocks;      /* persistent traversal blocks of 128 threads per SM (1..10;
+                                 the kernels fit 8, more is taken as 8) */
     int32_t material_sort;    /* 1: classify hits and shade per material class; 0: one kernel */
-    int32_t stack_smem;       /* traversal stack entries in shared memory: 16 or 32 */
+    int32_t stack_smem;       /* traversal stack entries per ray in shared memory:
+                                 32: 16 entries (default), 16: 8 entries */
     int32_t graphs;           /* 1: replay pairs of iterations as CUDA graphs */
     int32_t sample_film;      /* 1: batched renders write one record per sample and build the
                                  film from them afterwards (no film atomics; 16 bytes of HBM
                                  per sample, 24 with the Gaussian filter, whose film is then
                                  gathered per pixel from the records around it); 0: atomics */
-    int32_t spec_extend;      /* 1: closest-hit traversal lets a ray that holds a leaf keep
-                                 visiting inner nodes until it is blocked (speculative);
-                                 default 0 */
-    int32_t spec_shadow;      /* the same for the shadow (occlusion) traversal */
+    int32_t spec_extend;      /* 0 or 1; no effect (selected a speculative traversal that
+                                 was never faster) */
+    int32_t spec_shadow;      /* 0 or 1; no effect */
     int32_t ray_sort;         /* bit 0: before each closest-hit launch the active paths are
                                  reordered by a ray key (origin cell and direction bin) so
                                  that a warp's rays visit the same nodes; bit 1: the path
@@ -422,13 +421,13 @@ typedef struct gnd_tune {
     int32_t leaf_batch;       /* closest-hit traversal of renders (1..32): a warp leaves its
                                  inner-node phase for its leaf phase once this many of its
                                  rays hold a leaf; the others resume their traversal
-                                 afterwards (32: only when no ray can take another
-                                 inner-node step, the default) */
+                                 afterwards (16 and more: at 16, what one leaf pass
+                                 of a warp takes; default 32) */
     int32_t trace_leaf_batch; /* the same for the scene's ray batches (gnd_gpu_trace_*,
                                  except the _fixed form); default 12 */
     int32_t shadow_leaf_batch; /* the same for the path tracer's shadow queries; default 32 */
     int32_t trace_blocks;     /* persistent blocks of 128 threads per SM for the scene's ray
-                                 batches (1..10, as trav_blocks; default 8) */
+                                 batches (1..10; the kernels fit 8, more is taken as 8) */
 } gnd_tune;
 gnd_status gnd_gpu_get_tune(gnd_gpu_ctx* ctx, gnd_scene_id scene, gnd_tune* tune);
 gnd_status gnd_gpu_set_tune(gnd_gpu_ctx* ctx, gnd_scene_id scene, const gnd_tune* tune);

@@ -413,6 +413,7 @@ gnd_status gnd_gpu_scene_upload(gnd_gpu_ctx* ctxh, const gnd_scene_desc* d, gnd_
         for (int i = 0; i < d->num_instances; ++i) {
             const uint32_t t = mats[is[i].material].type;
             cls[i] = (uint8_t)(t < kMatIndex ? t : kMatIndex);
+            ds->matTypes |= 1u << cls[i];
             if (t == kMatIndex) { mask[i] = 1; ds->hasNullMaterials = true; }
         }
         ds->nullMask.alloc(mask.size());

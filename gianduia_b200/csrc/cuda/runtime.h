@@ -164,6 +164,7 @@ struct DeviceScene {
     int width = 0, height = 0, spp = 1, maxDepth = 1000, integrator = 0, filter = 0;
     float filterRadius[2] = {0.5f, 0.5f}, filterAlpha = 2.f;
     bool hasNullMaterials = false;
+    uint32_t matTypes = 0;    // material types of the instances (bit per MatType)
     int numMaterials = 0;
     Tune tune;                // engine settings for renders of this scene
     // array sizes (gnd_gpu_scene_info / gnd_gpu_scene_download)

@@ -103,7 +103,7 @@ __device__ __forceinline__ void blockAppend2(unsigned long long* pair, bool a, b
 }
 
 struct KParams {
-    const JobDev* jobs;
+    JobDev* jobs;
     PathState* paths;
     HitRec* hits;
     uint32_t* listIn;
@@ -129,6 +129,8 @@ struct KParams {
     uint32_t shadowLeafBatch;      // the same for the shadow queries
     uint32_t capacity;
     uint32_t fifo;                 // 1: grabs walk the active list from its first job
+    // the loop of the round's graph, when this is the last iteration of its body (0: none)
+    cudaGraphConditionalHandle loop;
 };
 
 // ---------------------------------------------------------------- surface interaction
@@ -774,29 +776,70 @@ __device__ __forceinline__ float generatePath(const JobDev& j, uint32_t jobIdx, 
     return time;
 }
 
-// ---------------------------------------------------------------- kernels
-__global__ void kBeginIter(KParams p) {
-    uint32_t* cnt = p.cnt;
+// ---------------------------------------------------------------- iteration control
+// One block of at least 32 threads: whether any active job has work items left to hand out,
+// after releasing the next pass of jobs that do so by themselves. No other block may be
+// handing out items.
+__device__ __forceinline__ bool workLeft(const KParams& p) {
+    const uint32_t na = *(volatile uint32_t*)&p.cnt[kQActive];
+    bool work = false;
+    for (uint32_t t = threadIdx.x; t < na; t += blockDim.x) {
+        const uint32_t jid = p.active[t];
+        JobDev& j = p.jobs[jid];
+        const unsigned long long next = *(volatile unsigned long long*)&p.ctl[jid].next;
+        unsigned long long end = *(volatile uint64_t*)&j.workEnd;
+        const unsigned long long pass = *(volatile uint64_t*)&j.passItems;
+        if (next >= end && pass && end < j.total) {
+            p.ctl[jid].next = end;   // a block's grab may have run past the end
+            end = min(end + pass, (unsigned long long)j.total);
+            j.workEnd = end;
+            work = true;
+        } else {
+            work = work || next < end;
+        }
+    }
+    return __syncthreads_or(work) != 0;
+}
+
+// Queue counters of the iteration to come: `in` active paths, `idle` slots on the free list.
+// Without work the idle slots are carried over unchanged: kRetire copies them to the front
+// of the next free list, reserved here.
+__device__ __forceinline__ void beginIteration(uint32_t* cnt, uint32_t in, uint32_t idle, bool work) {
+    cnt[kQIn] = in;
+    cnt[kQFree] = idle;
     cnt[kQOut] = 0;
     cnt[kQShadow] = 0;
     cnt[kQDone] = 0;
     cnt[kQFetchA] = 0;
     cnt[kQFetchB] = 0;
-    cnt[kQIter] += 1;   // iteration number: round-robin start of the job grabs
+    cnt[kQTicket] = 0;
     for (int k = 0; k < kShadeClasses; ++k) cnt[kQClass0 + k] = 0;
-    // Whether any active job has work items left to hand out (the hand-out limits change
-    // only between launches). Without work the idle slots are carried over unchanged:
-    // kRetire copies them to the front of the next free list, reserved here.
-    uint32_t work = 0;
-    const uint32_t na = cnt[kQActive];
-    for (uint32_t t = 0; t < na && !work; ++t) {
-        const uint32_t jid = p.active[t];
-        if (p.ctl[jid].next < p.jobs[jid].workEnd) work = 1;
-    }
-    cnt[kQWork] = work;
-    cnt[kQFreeOut] = work ? 0u : cnt[kQFree];
+    cnt[kQWork] = work ? 1u : 0u;
+    cnt[kQFreeOut] = work ? 0u : idle;
 }
 
+// Start of a round of at most `pairs` iteration pairs: the host may have admitted, released
+// or stopped jobs since the last one.
+__global__ void kBeginRound(KParams p, uint32_t pairs) {
+    const bool work = workLeft(p);
+    if (threadIdx.x != 0) return;
+    const uint32_t in = p.cnt[kQIn];
+    beginIteration(p.cnt, in, p.cnt[kQFree], work);
+    p.cnt[kQPairs] = pairs;
+    if (p.loop) cudaGraphSetConditional(p.loop, (in > 0 || work) ? 1u : 0u);
+}
+
+// End of a round: its counters into the host's snapshot (pinned memory).
+__global__ void kEndRound(KParams p, Wavefront::Snapshot* out) {
+    if (threadIdx.x < kMaxJobs) out->ctl[threadIdx.x] = p.ctl[threadIdx.x];
+    if (threadIdx.x != 0) return;
+    out->inflight = p.cnt[kQIn];
+    out->err = *p.errWord;
+    out->iterations = p.cnt[kQIter];
+    out->retiredAll = p.totals[2];
+}
+
+// ---------------------------------------------------------------- kernels
 // Shade class of a path after its extend query (see kMatClasses): volpath paths inside a
 // medium go to the medium class, others to their surface's class.
 static_assert(kMatIndex == kMatClasses - 1, "the null-BSDF material type is the last surface class");
@@ -1634,11 +1677,28 @@ __global__ void __launch_bounds__(kAggBlock, 3) kRetire(KParams p) {
         if (got) p.listOut[k] = slot;
         if (idle) p.freeOut[f] = slot;
     }
-}
-
-__global__ void kEndIter(uint32_t* cnt) {
-    cnt[kQIn] = cnt[kQOut];
-    cnt[kQFree] = cnt[kQFreeOut];
+    // the last block to get here prepares the next iteration (two one-thread launches per
+    // iteration before: 4 us of a 20 us iteration of a small image)
+    __shared__ bool sLast;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        sLast = atomicAdd(&p.cnt[kQTicket], 1u) == gridDim.x - 1u;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!sLast) return;
+    const bool left = workLeft(p);
+    if (threadIdx.x != 0) return;
+    volatile uint32_t* cnt = p.cnt;
+    const uint32_t in = cnt[kQOut], idle = cnt[kQFreeOut];
+    beginIteration(p.cnt, in, idle, left);
+    cnt[kQIter] = cnt[kQIter] + 1u;   // iteration number: round-robin start of the job grabs
+    if (p.loop) {
+        const uint32_t pairs = cnt[kQPairs] - 1u;
+        cnt[kQPairs] = pairs;
+        cudaGraphSetConditional(p.loop, (pairs > 0 && (in > 0 || left)) ? 1u : 0u);
+    }
 }
 
 // Fixed-point film -> float film [H*W][7] (sum wL rgb, sum w, sum wL^2 rgb).
@@ -1661,23 +1721,36 @@ __global__ void kResetPool(uint32_t* freeList, uint32_t n, uint32_t* cnt) {
     }
 }
 
-// One shade launch per material class of one integrator (empty classes exit at once).
+// One shade launch per shade class of one integrator that the admitted jobs can meet.
 template <bool VOL, bool EXT>
-static void launchShade(const KParams& kp, uint32_t* classLists, int grid, cudaStream_t st) {
+static void launchShade(const KParams& kp, uint32_t* classLists, uint32_t classes, int grid, cudaStream_t st) {
     const size_t cap = kp.capacity;
     const int c0 = VOL ? kClassesPerInt : 0;
+    classes >>= c0;
     uint32_t* cnt = kp.cnt + kQClass0 + c0;
     uint32_t* lists = classLists + (size_t)c0 * cap;
     static_assert(kMatMatte == 0 && kMatPlastic == 1 && kMatConductor == 2 && kMatGlass == 3,
                   "material classes follow the material type codes");
     // medium sampling first: its hand-offs join the surface classes shaded below
     if (VOL) kShade<true, kLobesNone, EXT><<<grid, kBlock, 0, st>>>(kp, lists + kMediumClass * cap, cnt + kMediumClass);
-    kShade<VOL, kLobesMatte, EXT><<<grid, kBlock, 0, st>>>(kp, lists + 0 * cap, cnt + 0);
-    kShade<VOL, kLobesPlastic, EXT><<<grid, kBlock, 0, st>>>(kp, lists + 1 * cap, cnt + 1);
-    kShade<VOL, kLobesConductor, EXT><<<grid, kBlock, 0, st>>>(kp, lists + 2 * cap, cnt + 2);
-    kShade<VOL, kLobesGlass, EXT><<<grid, kBlock, 0, st>>>(kp, lists + 3 * cap, cnt + 3);
-    kShade<VOL, kLobesAll, EXT><<<grid, kBlock, 0, st>>>(kp, lists + 4 * cap, cnt + 4);
+    if (classes & 1u) kShade<VOL, kLobesMatte, EXT><<<grid, kBlock, 0, st>>>(kp, lists + 0 * cap, cnt + 0);
+    if (classes & 2u) kShade<VOL, kLobesPlastic, EXT><<<grid, kBlock, 0, st>>>(kp, lists + 1 * cap, cnt + 1);
+    if (classes & 4u) kShade<VOL, kLobesConductor, EXT><<<grid, kBlock, 0, st>>>(kp, lists + 2 * cap, cnt + 2);
+    if (classes & 8u) kShade<VOL, kLobesGlass, EXT><<<grid, kBlock, 0, st>>>(kp, lists + 3 * cap, cnt + 3);
+    if (classes & 16u) kShade<VOL, kLobesAll, EXT><<<grid, kBlock, 0, st>>>(kp, lists + 4 * cap, cnt + 4);
 }
+
+// `path` jobs of a single material class (0..3): the class's kernel takes the active list as
+// it is and ends the escaped paths itself.
+template <bool EXT>
+static void launchShadeOne(const KParams& kp, uint32_t classes, int grid, cudaStream_t st) {
+    const uint32_t* n = kp.cnt + kQIn;
+    if (classes == 1u) kShade<false, kLobesMatte, EXT><<<grid, kBlock, 0, st>>>(kp, kp.listIn, n);
+    else if (classes == 2u) kShade<false, kLobesPlastic, EXT><<<grid, kBlock, 0, st>>>(kp, kp.listIn, n);
+    else if (classes == 4u) kShade<false, kLobesConductor, EXT><<<grid, kBlock, 0, st>>>(kp, kp.listIn, n);
+    else kShade<false, kLobesGlass, EXT><<<grid, kBlock, 0, st>>>(kp, kp.listIn, n);
+}
+static bool oneClass(uint32_t classes) { return classes == 1u || classes == 2u || classes == 4u || classes == 8u; }
 
 // ---------------------------------------------------------------- host driver
 Wavefront::Wavefront(Context* c) : ctx_(c) {
@@ -1799,7 +1872,7 @@ void Wavefront::syncActive() {
 }
 
 int Wavefront::admit(const DeviceScene& ds, int W, int H, int spp, int firstPass, int maxDepth, int integrator,
-                     const int window[4], uint64_t releaseItems) {
+                     const int window[4], uint64_t releaseItems, uint64_t passItems) {
     int j = -1;
     for (int k = 0; k < kMaxJobs; ++k)
         if (!jobs_[k].used) { j = k; break; }
@@ -1844,6 +1917,14 @@ int Wavefront::admit(const DeviceScene& ds, int W, int H, int spp, int firstPass
     hj.retired = 0;
     jd.workBegin = 0;
     jd.workEnd = hj.released;
+    jd.passItems = passItems;
+    jd.total = hj.total;
+    // class 4 (every lobe): null-BSDF surfaces, and escaped paths that are still shaded
+    // (shadeClass, ExtendSrc::store)
+    uint32_t cls = ds.matTypes & 15u;
+    if (ds.hasNullMaterials || integrator == 1 || ds.view.env.emitter >= 0) cls |= 16u;
+    if (integrator == 1) cls |= 1u << kMediumClass;
+    hj.classes = integrator == 1 ? cls << kClassesPerInt : cls;
     hj.used = true;
     hj.seq = seqNext_++;
     hj.prio = hj.seq;
@@ -1927,6 +2008,19 @@ void Wavefront::stop(int j) {
     HostJob& hj = jobs_[j];
     hj.dev.workEnd = 0;
     GND_CUDA(cudaMemsetAsync(&jobTab_.as<JobDev>()[j].workEnd, 0, sizeof(uint64_t), ctx_->stream));
+}
+
+void Wavefront::stopPasses(int j) {
+    HostJob& hj = jobs_[j];
+    hj.dev.passItems = 0;
+    GND_CUDA(cudaMemsetAsync(&jobTab_.as<JobDev>()[j].passItems, 0, sizeof(uint64_t), ctx_->stream));
+}
+
+uint32_t Wavefront::classes() const {
+    uint32_t c = 0;
+    for (const HostJob& j : jobs_)
+        if (j.used) c |= j.classes;
+    return c;
 }
 
 const float* Wavefront::resolvePinned(int j) {
@@ -2033,8 +2127,9 @@ void Wavefront::enqueueIteration(KParams kp, int par, int mix, bool hasNull, int
     kp.listOut = lists[par ^ 1];
     kp.freeIn = frees[par];
     kp.freeOut = frees[par ^ 1];
-    kBeginIter<<<1, 1, 0, st>>>(kp);
     kp.extList = kp.listIn;
+    const uint32_t cls = classes();
+    const uint32_t allPath = (1u << kClassesPerInt) - 1u;
     if (tune_.raySort & 1) {
         kRayKeys<false><<<grid, kBlock, 0, st>>>(kp);
         kRayScan<<<1, 1024, 0, st>>>(kp.rayBins);
@@ -2051,16 +2146,19 @@ void Wavefront::enqueueIteration(KParams kp, int par, int mix, bool hasNull, int
     }
     const bool count = (profile & 2) != 0;
     traversal(kp, mix, hasNull, count, st, ea, eb, 0);
-    if (sort) {
-        uint32_t* cls = classes_.as<uint32_t>();
-        kClassify<<<ctx_->numSMs * 4, kAggBlock, 0, st>>>(kp, cls);   // latency-bound: a full SM of warps
+    if (sort && mix == 1 && oneClass(cls & allPath)) {
+        if (ext_) launchShadeOne<true>(kp, cls, grid, st);
+        else launchShadeOne<false>(kp, cls, grid, st);
+    } else if (sort) {
+        uint32_t* lists = classes_.as<uint32_t>();
+        kClassify<<<ctx_->numSMs * 4, kAggBlock, 0, st>>>(kp, lists);   // latency-bound: a full SM of warps
         if (mix & 1) {
-            if (ext_) launchShade<false, true>(kp, cls, grid, st);
-            else launchShade<false, false>(kp, cls, grid, st);
+            if (ext_) launchShade<false, true>(kp, lists, cls, grid, st);
+            else launchShade<false, false>(kp, lists, cls, grid, st);
         }
         if (mix & 2) {
-            if (ext_) launchShade<true, true>(kp, cls, grid, st);
-            else launchShade<true, false>(kp, cls, grid, st);
+            if (ext_) launchShade<true, true>(kp, lists, cls, grid, st);
+            else launchShade<true, false>(kp, lists, cls, grid, st);
         }
     } else if (mix == 2) {
         if (ext_) kShade<true, kLobesAll, true><<<grid, kBlock, 0, st>>>(kp, kp.listIn, kp.cnt + kQIn);
@@ -2086,8 +2184,19 @@ void Wavefront::enqueueIteration(KParams kp, int par, int mix, bool hasNull, int
     // 12 blocks per SM: its register limit
     if (ext_) kRetire<true><<<ctx_->numSMs * 3, kAggBlock, 0, st>>>(kp);
     else kRetire<false><<<ctx_->numSMs * 3, kAggBlock, 0, st>>>(kp);
-    kEndIter<<<1, 1, 0, st>>>(kp.cnt);
     GND_CUDA(cudaGetLastError());
+}
+
+int Wavefront::launchesPerIteration(int mix) const {
+    const uint32_t cls = classes(), path = cls & ((1u << kClassesPerInt) - 1u);
+    const bool sort = tune_.sort != 0 || mix == 3;
+    int shade = 1;
+    if (sort && !(mix == 1 && oneClass(path))) {
+        shade = 1;   // classify
+        for (uint32_t c = cls; c; c &= c - 1u) ++shade;
+    }
+    return 2 + shade + (mix & 1 ? 1 : 0) + (mix & 2 ? 1 : 0) +   // extend and retire, shadow kernels
+           ((tune_.raySort & 1) ? 4 : 0) + ((tune_.raySort & 2) && (mix & 1) ? 4 : 0);
 }
 
 void Wavefront::clearGraphs() {
@@ -2095,27 +2204,56 @@ void Wavefront::clearGraphs() {
     graphs_.clear();
 }
 
-cudaGraphExec_t Wavefront::pairGraph(const KParams& kp, int par, int mix, bool hasNull, cudaStream_t st) {
+cudaGraphExec_t Wavefront::roundGraph(const KParams& kp, int par, int mix, bool hasNull, int pairs, cudaStream_t st) {
     const bool fifo = kp.fifo != 0;
+    const uint32_t cls = classes();
     for (const GraphEntry& g : graphs_)
-        if (g.par == par && g.mix == mix && g.hasNull == hasNull && g.fifo == fifo && g.motion == motion_ && g.ext == ext_)
+        if (g.par == par && g.mix == mix && g.pairs == pairs && g.classes == cls && g.hasNull == hasNull && g.fifo == fifo &&
+            g.motion == motion_ && g.ext == ext_)
             return g.exec;
-    cudaGraph_t graph = nullptr;
-    GND_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    if (graphs_.size() >= 64) clearGraphs();   // served mixes of scenes come and go
+    struct Guard {
+        cudaGraph_t g = nullptr;
+        ~Guard() {
+            if (g) cudaGraphDestroy(g);
+        }
+    } graph;
+    GND_CUDA(cudaGraphCreate(&graph.g, 0));
+    // kBeginRound -> while (loop) { two iterations }; the loop's value is set by kBeginRound and
+    // by the second iteration's kRetire. A turn of the loop costs 3.4 us beside its kernels.
+    KParams k = kp;
+    GND_CUDA(cudaGraphConditionalHandleCreate(&k.loop, graph.g, 0, cudaGraphCondAssignDefault));
+    uint32_t np = (uint32_t)pairs;
+    void* args[] = {&k, &np};
+    cudaKernelNodeParams kn{};
+    kn.func = reinterpret_cast<void*>(kBeginRound);
+    kn.gridDim = dim3(1);
+    kn.blockDim = dim3(kMaxJobs);
+    kn.kernelParams = args;
+    cudaGraphNode_t first, loop;
+    GND_CUDA(cudaGraphAddKernelNode(&first, graph.g, nullptr, 0, &kn));
+    cudaGraphNodeParams cn{};
+    cn.type = cudaGraphNodeTypeConditional;
+    cn.conditional.handle = k.loop;
+    cn.conditional.type = cudaGraphCondTypeWhile;
+    cn.conditional.size = 1;
+    GND_CUDA(cudaGraphAddNode(&loop, graph.g, &first, 1, &cn));
+    GND_CUDA(cudaStreamBeginCaptureToGraph(st, cn.conditional.phGraph_out[0], nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    cudaGraph_t body = nullptr;
     try {
-        enqueueIteration(kp, par, mix, hasNull, 0, st);
-        enqueueIteration(kp, par ^ 1, mix, hasNull, 0, st);
+        KParams a = kp;
+        a.loop = 0;
+        enqueueIteration(a, par, mix, hasNull, 0, st);
+        enqueueIteration(k, par ^ 1, mix, hasNull, 0, st);
     } catch (...) {
-        cudaStreamEndCapture(st, &graph);
-        if (graph) cudaGraphDestroy(graph);
+        cudaStreamEndCapture(st, &body);
         throw;
     }
-    GND_CUDA(cudaStreamEndCapture(st, &graph));
+    GND_CUDA(cudaStreamEndCapture(st, &body));
     cudaGraphExec_t exec = nullptr;
-    cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
-    cudaGraphDestroy(graph);
+    cudaError_t e = cudaGraphInstantiate(&exec, graph.g, 0);
     if (e != cudaSuccess) throw Error(GND_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-    graphs_.push_back(GraphEntry{par, mix, hasNull, fifo, motion_, ext_, exec});
+    graphs_.push_back(GraphEntry{par, mix, pairs, cls, hasNull, fifo, motion_, ext_, exec});
     return exec;
 }
 
@@ -2162,31 +2300,20 @@ void Wavefront::enqueueRound(int iters, int mix, bool hasNull, int profile, Resu
     kp.rayBins = rayBins_.as<uint32_t>();
     kp.raySorted = raySorted_.as<uint32_t>();
     kp.fifo = fifo_ ? 1u : 0u;
-    // begin, extend, retire, end; classify + 5 shade kernels per integrator when sorting (one
-    // shade kernel otherwise); 1 shadow kernel per integrator
-    const bool sort = tune_.sort != 0 || mix == 3;
-    const int nint = (mix & 1 ? 1 : 0) + (mix & 2 ? 1 : 0);
-    const int perIter = 4 + nint + (sort ? 1 + 5 * nint + ((mix & 2) ? 1 : 0) : 1) +   // + the medium kernel
-                        ((tune_.raySort & 1) ? 4 : 0) + ((tune_.raySort & 2) && (mix & 1) ? 4 : 0);
-    int it = 0;
-    while (it < iters) {
-        if (tune_.graphs && profile == 0 && iters - it >= 2) {
-            GND_CUDA(cudaGraphLaunch(pairGraph(kp, cur_, mix, hasNull, st), st));
-            it += 2;
-            acc.iterations += 2;
-            launches_ += 2 * perIter;
-        } else {
+    if (tune_.graphs && profile == 0 && iters >= 2 && !(iters & 1)) {
+        GND_CUDA(cudaGraphLaunch(roundGraph(kp, cur_, mix, hasNull, iters / 2, st), st));
+    } else {
+        kBeginRound<<<1, kMaxJobs, 0, st>>>(kp, 0u);
+        for (int it = 0; it < iters; ++it) {
             enqueueIteration(kp, cur_, mix, hasNull, profile, st);
             cur_ ^= 1;
-            ++it;
-            acc.iterations++;
-            launches_ += perIter;
         }
     }
-    GND_CUDA(cudaMemcpyAsync(&snaps_[slot].inflight, kp.cnt + kQIn, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    GND_CUDA(cudaMemcpyAsync(&snaps_[slot].err, kp.errWord, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    GND_CUDA(cudaMemcpyAsync(&snaps_[slot].retiredAll, kp.totals + 2, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    GND_CUDA(cudaMemcpyAsync(snaps_[slot].ctl, ctl_.ptr, kMaxJobs * sizeof(JobCtl), cudaMemcpyDeviceToHost, st));
+    kEndRound<<<1, kMaxJobs, 0, st>>>(kp, snaps_ + slot);
+    GND_CUDA(cudaGetLastError());
+    launches_ += 2;
+    perIter_ = launchesPerIteration(mix);
+    acc.iterations += iters;   // an upper bound: a round ends with its last path
     GND_CUDA(cudaEventRecord(snapEv_[slot], st));
 }
 
@@ -2213,7 +2340,9 @@ Wavefront::Result Wavefront::render(DeviceScene& ds, int W, int H, int spp, int 
         if (jobs_[j].used) throw Error(GND_ERR_INVALID, "the engine is serving jobs; render through the server");
     const uint64_t launches0 = launches_;
     reset(slots);
-    const int j = admit(ds, W, H, spp, firstPass, maxDepth, integrator, window, batched ? total : npix);
+    // plain renders without a callback: the device releases the passes
+    const bool devicePasses = !batched && !cb;
+    const int j = admit(ds, W, H, spp, firstPass, maxDepth, integrator, window, batched ? total : npix, devicePasses ? npix : 0);
     const int mix = integrator == 1 ? 2 : 1;
     // batched renders keep per-sample records instead of film atomics (at most 2^30
     // records: 16 GiB, and 8 GiB more of film positions with the Gaussian filter)
@@ -2233,9 +2362,9 @@ Wavefront::Result Wavefront::render(DeviceScene& ds, int W, int H, int spp, int 
     const int64_t iterCap = (int64_t)(maxDepth + 110) * (spp + 2) * 4 + 4096;
     bool cancelled = false;
     try {
-        if (batched) {
-            // every work item is released: rounds of kRoundIters iterations, one queued
-            // ahead of the one whose counters the host is reading
+        if (batched || devicePasses) {
+            // every work item is released, or the device releases them: rounds of kRoundIters
+            // iterations, one queued ahead of the one whose counters the host is reading
             const int kRoundIters = std::min(std::max(tune_.roundIters & ~1, 2), 64);
             int64_t k = 0, stopAt = -1;
             enqueueRound(kRoundIters, mix, ds.hasNullMaterials, profile, res, 0);
@@ -2248,20 +2377,21 @@ Wavefront::Result Wavefront::render(DeviceScene& ds, int W, int H, int spp, int 
                 // after a cancel, only rounds queued after the stop show the final state
                 if (cancelled && k > stopAt && inflight == 0) break;
                 if (c->cancel && !cancelled) {
-                    stop(j);            // queued behind round k + 1
+                    if (batched) stop(j);   // queued behind round k + 1
+                    else stopPasses(j);     // the passes released so far are finished
                     stopAt = k + 1;
                     cancelled = true;
                 }
-                if (res.iterations > iterCap) throw Error(GND_ERR_DEVICE_CHECK, "path iteration limit reached");
+                if ((int64_t)sn.iterations > iterCap) throw Error(GND_ERR_DEVICE_CHECK, "path iteration limit reached");
                 ++k;
             }
             GND_CUDA(cudaStreamSynchronize(st));   // the round queued ahead has nothing left to do
             if (records) filmFromSamples(j, total);
         }
-        while (!batched) {
+        while (!batched && !devicePasses) {
             uint32_t inflight = step(itersPerStep, mix, ds.hasNullMaterials, profile, res);
-            uint64_t r = retired(j);
-            if (!batched) {
+            uint64_t r = jobs_[j].retired;
+            {
                 while (pass < spp && r >= (uint64_t)(pass + 1) * npix) {
                     ++pass;
                     res.passesDone = pass;
@@ -2291,10 +2421,12 @@ Wavefront::Result Wavefront::render(DeviceScene& ds, int W, int H, int spp, int 
         drop(j);
         throw;
     }
-    if (batched) res.passesDone = cancelled ? (int)(retired(j) / std::max<uint64_t>(npix, 1)) : spp;
+    if (batched || devicePasses) res.passesDone = cancelled ? (int)(retired(j) / std::max<uint64_t>(npix, 1)) : spp;
     GND_CUDA(cudaEventRecord(e1, st));
     unsigned long long tot[8];
+    uint32_t iterations = 0;
     GND_CUDA(cudaMemcpyAsync(tot, totals_.ptr, sizeof(tot), cudaMemcpyDeviceToHost, st));
+    GND_CUDA(cudaMemcpyAsync(&iterations, counters_.as<uint32_t>() + kQIter, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     GND_CUDA(cudaStreamSynchronize(st));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
@@ -2323,7 +2455,8 @@ Wavefront::Result Wavefront::render(DeviceScene& ds, int W, int H, int spp, int 
     res.extendLeafSteps = (int64_t)tot[6];
     res.extendLeafWarpSteps = (int64_t)tot[7];
     res.ms = ms;
-    res.launches = (int64_t)(launches_ - launches0);
+    res.iterations = iterations;
+    res.launches = (int64_t)(launches_ - launches0) + res.iterations * perIter_;
     return res;
 }
 

@@ -55,6 +55,9 @@ struct JobDev {
     int32_t hasNull;
     int32_t firstPass;
     uint64_t workBegin, workEnd;   // work items [begin, end): item -> (pass, window pixel)
+    // Passes released by the device: when every item below workEnd is handed out, workEnd
+    // grows by passItems up to total (0: workEnd is the host's).
+    uint64_t passItems, total;
     // Per-sample film records (batched renders), indexed by work item; null: finished
     // samples are splatted into the film with atomics. With the Gaussian filter each
     // record also keeps its film position within its pixel (sampleOff).
@@ -67,7 +70,7 @@ struct JobDev {
 // both lists with a single atomic.
 enum QCounter : int {
     kQIn = 0, kQShadow = 2, kQDone = 3, kQFetchA = 4, kQFetchB = 5, kQFree = 6,
-    kQActive = 8, kQIter = 9, kQWork = 10, kQOut = 12, kQFreeOut = 13, kQClass0 = 16, kQCount = 32
+    kQActive = 8, kQIter = 9, kQWork = 10, kQTicket = 1, kQPairs = 7, kQOut = 12, kQFreeOut = 13, kQClass0 = 16, kQCount = 32
 };
 static_assert(kQOut % 2 == 0 && kQFreeOut == kQOut + 1, "kQOut / kQFreeOut must form an aligned pair");
 
@@ -90,12 +93,15 @@ struct HostJob {
     uint64_t bytes = 0;           // film bytes held in HBM
     uint64_t seq = 0;             // admission order
     uint64_t prio = 0;            // hand-out order key: lower first, ties by admission
+    uint32_t classes = 0;         // shade classes the job's paths can meet (bit per class)
 };
 
 // The engine: one pool of path slots shared by every admitted job. Each iteration runs
 // extend, shade, shadow and retire on the active list; retire splats finished samples
 // and refills their slots (and idle slots) with work items of the active jobs, taken
-// round-robin in warp-sized grabs.
+// round-robin in warp-sized grabs; its last block prepares the next iteration. A round is one
+// graph launch whose loop over iteration pairs runs on the device (conditional node) and
+// ends with the last path, so neither the host nor empty iterations stand between them.
 struct KParams;
 
 class Wavefront {
@@ -109,8 +115,9 @@ public:
         int passesDone = 0;
         double ms = 0.0, extendMs = 0.0;
     };
-    // One job to completion: plain = one pass in flight (the pool is one pass and each
-    // pass is released when the previous retired), batched = all passes released at once.
+    // One job to completion: plain = the pool is one pass and passes are released whole, one
+    // after another (on the device as slots free up; with a progress callback by the host when
+    // the previous pass has retired), batched = all passes released at once.
     // The film is added into filmHost (H x W x 7 floats) or, when fixedSum is given, in its
     // fixed-point form into fixedSum (H x W x 4 uint64) and fixedSq (H x W x 3 floats).
     Result render(DeviceScene& ds, int W, int H, int spp, int firstPass, int maxDepth, int integrator,
@@ -120,7 +127,7 @@ public:
     // ---- engine interface used by render() and by the server
     void reset(size_t slots);                         // (re)initialise the pool: every slot idle
     int admit(const DeviceScene& ds, int W, int H, int spp, int firstPass, int maxDepth, int integrator,
-              const int window[4], uint64_t releaseItems);
+              const int window[4], uint64_t releaseItems, uint64_t passItems = 0);
     void release(int job, uint64_t upTo);             // hand out work items [.., upTo)
     void finish(int job, float* filmHost);            // adds the film to filmHost, frees the job
     // adds the job's fixed-point sums into sum (H x W x 4) and sq (H x W x 3), frees the job
@@ -129,6 +136,7 @@ public:
     // The job's film resolved into pinned host memory (valid until the next call).
     const float* resolvePinned(int job);
     void stop(int job);                               // hands out no further work items of the job
+    void stopPasses(int job);                         // releases no further passes of the job
     void drop(int job);                               // frees the job without reading it
     // Runs `iters` iterations; returns the number of paths in flight afterwards.
     uint32_t step(int iters, int integratorMix, bool hasNull, int profile, Result& acc);
@@ -139,6 +147,8 @@ public:
     struct alignas(16) Snapshot {
         uint32_t inflight;            // active paths after the round
         uint32_t err;                 // the context's kernel error word after the round
+        uint32_t iterations;          // iterations since the pool was reset
+        uint32_t pad;
         unsigned long long retiredAll;   // paths retired by the engine since its pool was reset
         JobCtl ctl[kMaxJobs];         // per job: work items handed out, samples retired
     };
@@ -178,13 +188,16 @@ private:
     // One wavefront iteration on the stream for the lists of parity `par`.
     void enqueueIteration(KParams kp, int par, int mix, bool hasNull, int profile, cudaStream_t st);
     void traversal(const KParams& kp, int mix, bool hasNull, bool count, cudaStream_t st, cudaEvent_t ea, cudaEvent_t eb, int stage);
-    // Executable graph of two iterations (parity restored) for these settings, captured on
-    // first use; the per-iteration state it needs (queue counters, iteration number) is
-    // in device memory, so one capture serves every later replay.
-    cudaGraphExec_t pairGraph(const KParams& kp, int par, int mix, bool hasNull, cudaStream_t st);
+    // Executable graph of a round (at most `pairs` pairs of iterations, parity restored) for
+    // these settings, captured on first use; the per-iteration state it needs (queue
+    // counters, iteration number) is in device memory, so one capture serves every replay.
+    cudaGraphExec_t roundGraph(const KParams& kp, int par, int mix, bool hasNull, int pairs, cudaStream_t st);
+    int launchesPerIteration(int mix) const;
+    uint32_t classes() const;                         // shade classes of the admitted jobs
     void clearGraphs();
     struct GraphEntry {
-        int par, mix;
+        int par, mix, pairs;
+        uint32_t classes;
         bool hasNull, fifo, motion, ext;
         cudaGraphExec_t exec;
     };
@@ -201,7 +214,8 @@ private:
     Snapshot* snaps_ = nullptr;       // pinned host memory, two slots
     cudaEvent_t snapEv_[2] = {nullptr, nullptr};
     bool fifo_ = false;
-    uint64_t launches_ = 0;           // kernels launched by the engine so far
+    uint64_t launches_ = 0;           // kernels launched by the engine so far, outside iterations
+    int perIter_ = 0;                 // kernels of one iteration of the last round
     uint64_t seqNext_ = 0;
     HostJob jobs_[kMaxJobs];
     std::vector<cudaEvent_t> evs_;    // profile: (start, end) of each extend launch, from evPool_

@@ -136,6 +136,32 @@ __global__ void kValidateNodes(const Node4* __restrict__ nodes, int64_t n, int64
     if (f && (threadIdx.x & 31) == 0) atomicOr(flags, f);
 }
 
+// Texture bucket of every material (SceneView::instBucket): materials whose slots hold the
+// same kinds of texture trees share one; 0: no trees. Beyond 31 kinds of material
+// the buckets wrap, which only mixes some warps.
+std::vector<uint8_t> textureBuckets(const gnd_scene_desc* d) {
+    std::vector<uint8_t> out((size_t)std::max(d->num_materials, 0), 0);
+    const Material* mats = reinterpret_cast<const Material*>(d->materials);
+    const TexNode* nodes = reinterpret_cast<const TexNode*>(d->tex_nodes);
+    std::map<std::vector<int32_t>, int> seen;
+    for (int m = 0; m < d->num_materials; ++m) {
+        std::vector<int32_t> kinds;
+        bool any = false;
+        auto slot = [&](const ColorTex& t) {
+            kinds.push_back(t.kind == kTexNode ? 2 + nodes[t.node].kind : 0);
+            any = any || t.kind == kTexNode;
+        };
+        slot(mats[m].a);
+        slot(mats[m].b);
+        for (uint32_t r : {mats[m].roughTex, mats[m].etaTex, mats[m].kTex, mats[m].normalTex, mats[m].bumpTex}) {
+            kinds.push_back(r ? 2 + nodes[r - 1].kind : 0);
+            any = any || r;
+        }
+        if (any) out[m] = (uint8_t)(1 + seen.emplace(kinds, (int)seen.size()).first->second % (kTexBuckets - 1));
+    }
+    return out;
+}
+
 template <typename T>
 const T* upload(DeviceScene& ds, cudaStream_t st, const void* src, size_t count) {
     size_t bytes = count * sizeof(T);
@@ -410,10 +436,13 @@ gnd_status gnd_gpu_scene_upload(gnd_gpu_ctx* ctxh, const gnd_scene_desc* d, gnd_
         // null-BSDF mask and material type per instance
         std::vector<uint8_t> mask(std::max(1, d->num_instances), 0), cls(std::max(1, d->num_instances), kMatIndex);
         const Material* mats = reinterpret_cast<const Material*>(d->materials);
+        const std::vector<uint8_t> buckets = d->num_tex_nodes > 0 ? textureBuckets(d) : std::vector<uint8_t>();
+        std::vector<uint8_t> bucket(d->num_tex_nodes > 0 ? (size_t)d->num_instances : 0, 0);
         for (int i = 0; i < d->num_instances; ++i) {
             const uint32_t t = mats[is[i].material].type;
             cls[i] = (uint8_t)(t < kMatIndex ? t : kMatIndex);
             ds->matTypes |= 1u << cls[i];
+            if (!bucket.empty()) bucket[i] = buckets[is[i].material];
             if (t == kMatIndex) { mask[i] = 1; ds->hasNullMaterials = true; }
         }
         ds->nullMask.alloc(mask.size());
@@ -421,6 +450,7 @@ gnd_status gnd_gpu_scene_upload(gnd_gpu_ctx* ctxh, const gnd_scene_desc* d, gnd_
         ds->instClass.alloc(cls.size());
         GND_CUDA(cudaMemcpyAsync(ds->instClass.ptr, cls.data(), cls.size(), cudaMemcpyHostToDevice, st));
         v.instClass = ds->instClass.as<uint8_t>();
+        v.instBucket = bucket.empty() ? nullptr : upload<uint8_t>(*ds, st, bucket.data(), bucket.size());
         ds->viewDev.alloc(sizeof(SceneView));
         GND_CUDA(cudaMemcpyAsync(ds->viewDev.ptr, &v, sizeof(SceneView), cudaMemcpyHostToDevice, st));
         GND_CUDA(cudaStreamSynchronize(st));

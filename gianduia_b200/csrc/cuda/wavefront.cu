@@ -988,37 +988,63 @@ __global__ void __launch_bounds__(kBlock) kRayScatter(KParams p) {
 
 // Active list -> per-class lists (and kClassDone -> the done list): per block, the warps'
 // groups of one class take consecutive places (shared-memory counts), then one atomic per
-// class per block.
+// class per block. BUCKETS (scenes with textures): within the block's share of a class the
+// paths are grouped by their texture bucket, so that a shade warp mostly evaluates one kind
+// of texture (textured box, 640x360x16: matte shade kernel 10.6 -> 24.5 lanes per instruction,
+// 625 -> 442 us on 8 passes).
+template <bool BUCKETS>
 __global__ void __launch_bounds__(kAggBlock, 4) kClassify(KParams p, uint32_t* classLists) {
     constexpr int kLists = kShadeClasses + 1;   // the class lists and the done list
-    __shared__ uint32_t sCount[kLists], sBase[kLists];
+    constexpr int kBuckets = BUCKETS ? kTexBuckets : 1;
+    static_assert(kBuckets == 1 || (kBuckets == 32 && kLists <= kAggWarps), "a warp per list, a lane per bucket");
+    __shared__ uint32_t sCount[kLists * kBuckets], sBase[kLists * kBuckets];
     const uint32_t n = p.cnt[kQIn];
     const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t bb = blockIdx.x * kAggBlock; bb < n; bb += gridDim.x * kAggBlock) {   // block-uniform
         const uint32_t i = bb + threadIdx.x;
         const bool valid = i < n;
-        uint32_t cls = 0xFFFFFFFFu, slot = 0;
+        uint32_t cls = 0, key = 0xFFFFFFFFu, slot = 0;
         if (valid) {
             slot = p.listIn[i];
-            cls = p.hits[slot].pad[0];   // written by the extend store (shadeClass or kClassDone)
+            key = cls = p.hits[slot].pad[0];   // written by the extend store (shadeClass or kClassDone)
+            if (BUCKETS) {
+                const int inst = p.hits[slot].inst;
+                const uint8_t* bucket = p.jobs[p.paths[slot].flags >> 8].view.instBucket;
+                key = cls * kBuckets + (inst >= 0 && bucket ? (uint32_t)__ldg(bucket + inst) : 0u);
+            }
         }
         __syncthreads();   // the previous iteration's reads of sBase are over
-        if (threadIdx.x < (unsigned)kLists) sCount[threadIdx.x] = 0;
+        if (threadIdx.x < (unsigned)(kLists * kBuckets)) sCount[threadIdx.x] = 0;
         __syncthreads();
-        const uint32_t grp = __match_any_sync(0xffffffffu, cls);
+        const uint32_t grp = __match_any_sync(0xffffffffu, key);
         const int leader = __ffs(grp) - 1;
         uint32_t off = 0;
-        if (valid && (int)lane == leader) off = atomicAdd(&sCount[cls], (uint32_t)__popc(grp));
+        if (valid && (int)lane == leader) off = atomicAdd(&sCount[key], (uint32_t)__popc(grp));
         off = __shfl_sync(0xffffffffu, off, leader);
         __syncthreads();
-        if (threadIdx.x < (unsigned)kLists) {
+        if (BUCKETS) {
+            const uint32_t list = threadIdx.x >> 5;   // warp-uniform
+            if (list < (uint32_t)kLists) {
+                const uint32_t c = sCount[list * kBuckets + lane];
+                uint32_t incl = c;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+                    if ((int)lane >= o) incl += v;
+                }
+                const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+                uint32_t base = 0;
+                if (lane == 0 && total)
+                    base = atomicAdd(list < (uint32_t)kShadeClasses ? &p.cnt[kQClass0 + list] : &p.cnt[kQDone], total);
+                sBase[list * kBuckets + lane] = __shfl_sync(0xffffffffu, base, 0) + incl - c;
+            }
+        } else if (threadIdx.x < (unsigned)kLists) {
             const uint32_t c = sCount[threadIdx.x];
             uint32_t* counter = threadIdx.x < (unsigned)kShadeClasses ? &p.cnt[kQClass0 + threadIdx.x] : &p.cnt[kQDone];
             sBase[threadIdx.x] = c ? atomicAdd(counter, c) : 0u;
         }
         __syncthreads();
         if (valid) {
-            const uint32_t at = sBase[cls] + off + (uint32_t)__popc(grp & ((1u << lane) - 1u));
+            const uint32_t at = sBase[key] + off + (uint32_t)__popc(grp & ((1u << lane) - 1u));
             if (cls < (uint32_t)kShadeClasses) classLists[(size_t)cls * p.capacity + at] = slot;
             else p.done[at] = slot;
         }
@@ -1032,8 +1058,9 @@ __global__ void __launch_bounds__(kAggBlock, 4) kClassify(KParams p, uint32_t* c
 // class (medium sampling marked done) for a surface kernel later in the iteration.
 // EXT: some job of the launch uses the rarer features (SceneView::ext); without them the
 // kernel keeps the area-light, static-transform code only.
+// 128 registers (4 blocks per SM); the all-lobe kernels, which few paths take, up to 255.
 template <bool VOL, uint32_t M, bool EXT>
-__global__ void __launch_bounds__(kBlock) kShade(KParams p, const uint32_t* list, const uint32_t* count) {
+__global__ void __launch_bounds__(kBlock, M == kLobesAll ? 2 : 4) kShade(KParams p, const uint32_t* list, const uint32_t* count) {
     const uint32_t n = *count;
     for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
         uint32_t slot = list[i];
@@ -2146,12 +2173,14 @@ void Wavefront::enqueueIteration(KParams kp, int par, int mix, bool hasNull, int
     }
     const bool count = (profile & 2) != 0;
     traversal(kp, mix, hasNull, count, st, ea, eb, 0);
-    if (sort && mix == 1 && oneClass(cls & allPath)) {
+    if (sort && mix == 1 && oneClass(cls & allPath) && !textured_) {
         if (ext_) launchShadeOne<true>(kp, cls, grid, st);
         else launchShadeOne<false>(kp, cls, grid, st);
     } else if (sort) {
         uint32_t* lists = classes_.as<uint32_t>();
-        kClassify<<<ctx_->numSMs * 4, kAggBlock, 0, st>>>(kp, lists);   // latency-bound: a full SM of warps
+        // latency-bound: a full SM of warps
+        if (textured_) kClassify<true><<<ctx_->numSMs * 4, kAggBlock, 0, st>>>(kp, lists);
+        else kClassify<false><<<ctx_->numSMs * 4, kAggBlock, 0, st>>>(kp, lists);
         if (mix & 1) {
             if (ext_) launchShade<false, true>(kp, lists, cls, grid, st);
             else launchShade<false, false>(kp, lists, cls, grid, st);
@@ -2191,7 +2220,7 @@ int Wavefront::launchesPerIteration(int mix) const {
     const uint32_t cls = classes(), path = cls & ((1u << kClassesPerInt) - 1u);
     const bool sort = tune_.sort != 0 || mix == 3;
     int shade = 1;
-    if (sort && !(mix == 1 && oneClass(path))) {
+    if (sort && !(mix == 1 && oneClass(path) && !textured_)) {
         shade = 1;   // classify
         for (uint32_t c = cls; c; c &= c - 1u) ++shade;
     }
@@ -2209,7 +2238,7 @@ cudaGraphExec_t Wavefront::roundGraph(const KParams& kp, int par, int mix, bool 
     const uint32_t cls = classes();
     for (const GraphEntry& g : graphs_)
         if (g.par == par && g.mix == mix && g.pairs == pairs && g.classes == cls && g.hasNull == hasNull && g.fifo == fifo &&
-            g.motion == motion_ && g.ext == ext_)
+            g.motion == motion_ && g.ext == ext_ && g.textured == textured_)
             return g.exec;
     if (graphs_.size() >= 64) clearGraphs();   // served mixes of scenes come and go
     struct Guard {
@@ -2253,7 +2282,7 @@ cudaGraphExec_t Wavefront::roundGraph(const KParams& kp, int par, int mix, bool 
     cudaGraphExec_t exec = nullptr;
     cudaError_t e = cudaGraphInstantiate(&exec, graph.g, 0);
     if (e != cudaSuccess) throw Error(GND_ERR_CUDA, std::string("cudaGraphInstantiate: ") + cudaGetErrorString(e));
-    graphs_.push_back(GraphEntry{par, mix, pairs, cls, hasNull, fifo, motion_, ext_, exec});
+    graphs_.push_back(GraphEntry{par, mix, pairs, cls, hasNull, fifo, motion_, ext_, textured_, exec});
     return exec;
 }
 
@@ -2275,10 +2304,12 @@ void Wavefront::enqueueRound(int iters, int mix, bool hasNull, int profile, Resu
     cudaStream_t st = c->stream;
     motion_ = false;   // the traversal variant for animated instances, when a job needs it
     ext_ = false;      // the shade / retire variants for the rarer features
+    textured_ = false; // a job's scene has texture trees
     for (int j = 0; j < kMaxJobs; ++j) {
         if (!jobs_[j].used) continue;
         if (jobs_[j].dev.view.motion) motion_ = true;
         if (jobs_[j].dev.view.ext) ext_ = true;
+        if (jobs_[j].dev.view.numTexNodes > 0) textured_ = true;
     }
     KParams kp{};
     kp.jobs = jobTab_.as<JobDev>();

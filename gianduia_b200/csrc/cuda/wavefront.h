@@ -198,11 +198,12 @@ private:
     struct GraphEntry {
         int par, mix, pairs;
         uint32_t classes;
-        bool hasNull, fifo, motion, ext;
+        bool hasNull, fifo, motion, ext, textured;
         cudaGraphExec_t exec;
     };
     bool motion_ = false;   // an admitted job's scene has animated instances (MOTION traversal)
     bool ext_ = false;      // an admitted job's scene uses the EXT features (SceneView::ext)
+    bool textured_ = false; // an admitted job's scene has texture trees
     std::vector<GraphEntry> graphs_;
     Tune tune_;
     Context* ctx_;

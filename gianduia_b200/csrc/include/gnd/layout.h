@@ -241,6 +241,7 @@ struct alignas(16) Camera {
 static_assert(sizeof(Camera) == 320, "Camera record must be 320 bytes");
 
 // ---------------------------------------------------------------- scene view
+constexpr int kTexBuckets = 32;   // SceneView::instBucket
 // Device pointers of one uploaded scene, passed by value to kernels (or read from an
 // array of views when several scenes share one launch).
 struct SceneView {
@@ -257,6 +258,8 @@ struct SceneView {
     const float* cdf;
     const uint32_t* origToLeaf;
     const uint8_t* instClass;     // per instance: material type, kMatIndex for null-BSDF ones
+    const uint8_t* instBucket;    // per instance: bucket (below kTexBuckets) of the textures its material
+                                  // evaluates, 0 without any; null for scenes without texture trees
     const InstMotion* motion;     // per instance, read for instances flagged kInstAnimated
     const TexNode* texNodes;      // texture trees (ColorTex kind kTexNode)
     const float* texels;          // image texture texels, 4 floats (rgba) each

@@ -30,7 +30,6 @@ struct THit {
 
 enum TraceError : int { kTraceOk = 0, kTraceStackOverflow = 1, kTraceIterLimit = 2, kTraceBadRef = 4 };
 
-constexpr int kStackSize = 64;
 constexpr uint32_t kSentinel = 0xFFFFFFFEu;
 constexpr uint32_t kMaxIterations = 1u << 22;
 
@@ -145,151 +144,9 @@ __device__ __forceinline__ void animatedW2ORows(const SceneView& s, uint32_t id,
     r2 = make_float4(w.r[2][0], w.r[2][1], w.r[2][2], w.r[2][3]);
 }
 
-// Trace one ray to its closest hit. `stk` points at this thread's first stack entry in
-// shared memory; entries are BLOCK apart. Returns an error bitmask (0 on success).
-template <int BLOCK, bool MOTION = false>
-__device__ __forceinline__ int traceRay(const SceneView& s, const TRay& ray, THit& hit, uint32_t* stk) {
-    hit.t = INFINITY;
-    hit.u = hit.v = 0.f;
-    hit.inst = -1;
-    hit.slot = 0xFFFFFFFFu;
-    if (s.tlasRoot == kEmpty || missesAll(s, ray)) return kTraceOk;
-    const V3 wo = ray.o, wd = ray.d;
-    const float wtmin = ray.tmin;
-    float tmax = ray.tmax;          // shrinks with every accepted hit
-    float bestT = 3.402823466e38f;  // bvh.cpp:39 (FLT_MAX)
-    V3 o = wo, d = wd;
-    V3 inv = v3(__frcp_rn(wd.x), __frcp_rn(wd.y), __frcp_rn(wd.z));
-    float tmin = wtmin;
-    int curInst = -1;
-    int sp = 0;
-    stk[0] = s.tlasRoot;
-    sp = 1;
-    uint32_t iter = 0;
-    int err = 0;
-    while (sp > 0) {
-        if (++iter > kMaxIterations) { err |= kTraceIterLimit; break; }
-        uint32_t e = stk[(--sp) * BLOCK];
-        if (e == kSentinel) {
-            // leave the bottom-level tree: back to the world-space ray
-            o = wo; d = wd;
-            inv = v3(__frcp_rn(wd.x), __frcp_rn(wd.y), __frcp_rn(wd.z));
-            tmin = wtmin;
-            curInst = -1;
-            continue;
-        }
-        if (!isLeaf(e)) {
-            const Node4* nd = s.nodes + e;
-            float4 lx = ldg4(nd->lox), hx = ldg4(nd->hix), ly = ldg4(nd->loy);
-            float4 hy = ldg4(nd->hiy), lz = ldg4(nd->loz), hz = ldg4(nd->hiz);
-            uint4 ch = ldgu4(nd->child);
-            float key[4];
-            uint32_t ref[4] = {ch.x, ch.y, ch.z, ch.w};
-            const float LX[4] = {lx.x, lx.y, lx.z, lx.w}, HX[4] = {hx.x, hx.y, hx.z, hx.w};
-            const float LY[4] = {ly.x, ly.y, ly.z, ly.w}, HY[4] = {hy.x, hy.y, hy.z, hy.w};
-            const float LZ[4] = {lz.x, lz.y, lz.z, lz.w}, HZ[4] = {hz.x, hz.y, hz.z, hz.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                float t1x = (LX[i] - o.x) * inv.x, t2x = (HX[i] - o.x) * inv.x;
-                float t1y = (LY[i] - o.y) * inv.y, t2y = (HY[i] - o.y) * inv.y;
-                float t1z = (LZ[i] - o.z) * inv.z, t2z = (HZ[i] - o.z) * inv.z;
-                float tn = lmax(lmax(lmin(t1x, t2x), lmin(t1y, t2y)), lmax(lmin(t1z, t2z), tmin));
-                float tf = lmin(lmin(lmax(t1x, t2x), lmax(t1y, t2y)), lmin(lmax(t1z, t2z), tmax));
-                key[i] = (tn <= tf && ref[i] != kEmpty) ? tn : INFINITY;
-            }
-            // ascending sort network on (key, ref)
-#define GND_CSWAP(a, b)                                                          \
-    if (key[b] < key[a]) {                                                       \
-        float tk = key[a]; key[a] = key[b]; key[b] = tk;                         \
-        uint32_t tr = ref[a]; ref[a] = ref[b]; ref[b] = tr;                      \
-    }
-            GND_CSWAP(0, 1) GND_CSWAP(2, 3) GND_CSWAP(0, 2) GND_CSWAP(1, 3) GND_CSWAP(1, 2)
-#undef GND_CSWAP
-#pragma unroll
-            for (int i = 3; i >= 0; --i) {
-                if (key[i] != INFINITY) {
-                    if (sp >= kStackSize) { err |= kTraceStackOverflow; break; }
-                    stk[(sp++) * BLOCK] = ref[i];
-                }
-            }
-            if (err) break;
-            continue;
-        }
-        // leaf
-        uint32_t first = leafFirst(e), count = leafCount(e);
-        if (curInst >= 0) {
-            // bottom level: triangles [first, first + count)
-            for (uint32_t k = 0; k < count; ++k) {
-                float t, u, v;
-                uint32_t prim;
-                if (triTest(s.tris + first + k, o, d, tmin, tmax, t, u, v, prim)) {
-                    tmax = t;
-                    bestT = t;
-                    hit.t = t; hit.u = u; hit.v = v;
-                    hit.inst = curInst;
-                    hit.slot = first + k;
-                }
-            }
-            continue;
-        }
-        // top level: instances tlasList[first .. first + count)
-        for (uint32_t k = 0; k < count; ++k) {
-            uint32_t id = __ldg(s.tlasList + first + k);
-            const InstTrav* it = s.instT + id;
-            float4 r0 = ldg4(&it->w2o.r[0][0]), r1 = ldg4(&it->w2o.r[1][0]), r2 = ldg4(&it->w2o.r[2][0]);
-            float4 meta = ldg4(&it->kind);
-            uint32_t kind = __float_as_uint(meta.x);
-            if (MOTION && (kind & kInstAnimated)) animatedW2ORows(s, id, ray.time, r0, r1, r2);
-            kind &= ~kInstAnimated;
-            // primitive.cpp:49-50: rLocal = worldToObject(rWorld), tMin = Epsilon
-            V3 lo, ld;
-            lo.x = (r0.x * wo.x + r0.y * wo.y) + (r0.z * wo.z + r0.w);
-            lo.y = (r1.x * wo.x + r1.y * wo.y) + (r1.z * wo.z + r1.w);
-            lo.z = (r2.x * wo.x + r2.y * wo.y) + (r2.z * wo.z + r2.w);
-            ld.x = (r0.x * wd.x + r0.y * wd.y) + (r0.z * wd.z + r0.w * 0.0f);
-            ld.y = (r1.x * wd.x + r1.y * wd.y) + (r1.z * wd.z + r1.w * 0.0f);
-            ld.z = (r2.x * wd.x + r2.y * wd.y) + (r2.z * wd.z + r2.w * 0.0f);
-            if (kind == kShapeMesh) {
-                uint32_t root = __float_as_uint(meta.y);
-                if (root == kEmpty) continue;
-                // remaining instances of this leaf come back after the bottom level
-                if (k + 1 < count) {
-                    if (sp >= kStackSize) { err |= kTraceStackOverflow; break; }
-                    stk[(sp++) * BLOCK] = makeLeaf(first + k + 1, count - k - 1);
-                }
-                if (sp + 2 > kStackSize) { err |= kTraceStackOverflow; break; }
-                stk[(sp++) * BLOCK] = kSentinel;
-                stk[(sp++) * BLOCK] = root;
-                o = lo; d = ld;
-                inv = v3(__frcp_rn(ld.x), __frcp_rn(ld.y), __frcp_rn(ld.z));
-                tmin = kEpsilon;
-                curInst = (int)id;
-                break;
-            }
-            float th;
-            bool h;
-            if (kind == kShapeSphere) {
-                h = sphereTest(meta.z, lo, ld, kEpsilon, tmax, th);
-            } else {
-                float ez = __ldg(&s.instS[id].ext[2]);
-                h = cubeTest(v3(meta.z, meta.w, ez), lo, ld, kEpsilon, tmax, th);
-            }
-            if (h && th < bestT) {
-                tmax = th;
-                bestT = th;
-                hit.t = th; hit.u = 0.f; hit.v = 0.f;
-                hit.inst = (int)id;
-                hit.slot = 0xFFFFFFFFu;
-            }
-        }
-        if (err) break;
-    }
-    return err;
-}
-
 // ---------------------------------------------------------------- persistent traversal
-// The same traversal as traceRay, restated as an incremental per-lane state machine for
-// persistent warps: lanes that finish a ray fetch the next one (warp-aggregated atomic on
+// Traversal as an incremental per-lane state machine (traceOne below runs it for one ray per
+// thread) for persistent warps: lanes that finish a ray fetch the next one (warp-aggregated atomic on
 // a per-launch counter), and each round runs a node phase (every lane tests inner nodes
 // until it holds a leaf) and a leaf pass (the warp's lanes share out the pending triangles),
 // so the warp executes one code path at a time.
@@ -724,6 +581,57 @@ __device__ __forceinline__ uint32_t warpFetch(uint32_t* counter, bool want) {
         base = __shfl_sync(0xffffffffu, base, leader);
     }
     return base + (uint32_t)__popc(mask & ((1u << lane) - 1u));
+}
+
+// One ray per thread to its closest hit (the transmittance queries: a few short segments each,
+// in small scenes; a thread's own loop costs less than the persistent loop's phases there).
+struct OneRay {
+    const TRay* r;
+    __device__ __forceinline__ void world(V3& o, V3& d, float& tmin) const { o = r->o; d = r->d; tmin = r->tmin; }
+};
+template <bool MOTION, int BLOCK, int SMEM>
+__device__ __forceinline__ int traceOne(const SceneView& s, const TRay& ray, THit& hit, TStack<BLOCK, SMEM, true>& st) {
+    Trav t;
+    const OneRay src{&ray};
+    travInit(t, s, ray);
+    if (!t.fast && missesAll(s, ray)) t.cur = kEmpty;
+    const Node4* nodes = s.nodes;
+    int err = 0;
+    uint32_t iter = 0;
+    while (t.cur != kEmpty || t.leaf != kEmpty) {
+        while (t.cur != kEmpty) {
+            const int e = travNodeStep<false, true, true>(t, nodes, st, src, nullptr);
+            if (e || ++iter > kMaxIterations) {
+                err |= e ? e : (int)kTraceIterLimit;
+                travStop(t);
+            }
+        }
+        if (t.leaf == kEmpty) break;   // the stack is empty
+        if (t.curInst >= 0) {
+            const uint32_t first = leafFirst(t.leaf), count = leafCount(t.leaf);
+            for (uint32_t k = 0; k < count; ++k) {
+                float tt, u, v;
+                uint32_t prim;
+                if (triTest(s.tris + first + k, t.o, t.d, t.tmin, t.tmax, tt, u, v, prim)) {
+                    t.tmax = tt;
+                    t.u = u; t.v = v;
+                    t.inst = t.curInst;
+                    t.slot = first + k;
+                }
+            }
+            travPop<true>(t, st, src);
+        } else {
+            const int e = travInstStep<false, MOTION>(t, s, st, nullptr, ray.time);
+            if (e) {
+                err |= e;
+                travStop(t);
+            } else if (t.cur == kEmpty && t.leaf == kEmpty) {
+                travPop<true>(t, st, src);
+            }
+        }
+    }
+    hit = travHit(t);
+    return err;
 }
 
 // Persistent traversal loop. Every lane of every warp runs it to the end (the block size

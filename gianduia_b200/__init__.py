@@ -329,8 +329,9 @@ class GpuContext:
         post_params."""
         a = np.ascontiguousarray(rgb, dtype=np.float32)
         h, w = a.shape[:2]
-        hdr = np.zeros((h, w, 3), np.float32) if want_hdr else None
-        out8 = np.zeros((h, w, 3), np.uint8) if want_rgb8 else None
+        # outputs that a call writes whole are not cleared first (a 12 MB image: 0.7 ms)
+        hdr = np.empty((h, w, 3), np.float32) if want_hdr else None
+        out8 = np.empty((h, w, 3), np.uint8) if want_rgb8 else None
         p = post_params(**params)
         _check(lib().gnd_gpu_post(self._h, a.ctypes.data, w, h, ctypes.byref(p),
                                   hdr.ctypes.data if hdr is not None else None,
@@ -370,15 +371,15 @@ class GpuContext:
 
     def trace_closest(self, sid, rays):
         r = as_rays(rays)
-        hits = np.zeros(r.shape[0], HIT_DTYPE)
+        hits = np.empty(r.shape[0], HIT_DTYPE)
         _check(lib().gnd_gpu_trace_closest(self._h, sid, r.ctypes.data, r.shape[0], hits.ctypes.data), "gnd_gpu_trace_closest")
         return hits
 
     def trace_any(self, sid, rays):
         r = as_rays(rays)
-        occ = np.zeros(r.shape[0], np.uint8)
+        occ = np.empty(r.shape[0], np.uint8)
         _check(lib().gnd_gpu_trace_any(self._h, sid, r.ctypes.data, r.shape[0], occ.ctypes.data), "gnd_gpu_trace_any")
-        return occ.astype(bool)
+        return occ.view(np.bool_)   # the kernel writes 0 or 1
 
     # device-pointer variants (pointers as ints, e.g. torch tensor.data_ptr())
     def trace_closest_dev(self, sid, d_rays, n, d_hits, stream=0):
@@ -526,7 +527,7 @@ class GpuContext:
         """Blocks until the job finishes; returns (film [H, W, 7], status dict). A cancelled
         or failed job raises GndError; wait_any returns its status code instead."""
         h, w = self._jobs[jid]
-        film = np.zeros((h, w, 7), np.float32)
+        film = np.empty((h, w, 7), np.float32)   # written whole, or the call raises
         st = JobStatus()
         _check(lib().gnd_gpu_serve_wait(self._h, jid, film.ctypes.data, ctypes.byref(st), int(timeout_ms)),
                "gnd_gpu_serve_wait")

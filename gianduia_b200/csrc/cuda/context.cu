@@ -4,6 +4,7 @@
 
 #include "bvhbuild.h"
 #include "runtime.h"
+#include "hostcopy.h"
 #include "server.h"
 #include "wavefront.h"
 
@@ -15,6 +16,12 @@ thread_local std::string t_lastError = "no error";
 void setLastError(const std::string& m) { t_lastError = m; }
 const std::string& lastError() { return t_lastError; }
 
+Context::Context() = default;
+HostCopy& Context::copies() {
+    if (!hostCopy) hostCopy = std::make_unique<HostCopy>(device);
+    return *hostCopy;
+}
+
 Context::~Context() {
     if (device >= 0) cudaSetDevice(device);
     server.reset();   // joins the serving thread before the engine goes away
@@ -22,6 +29,7 @@ Context::~Context() {
     scenes.clear();
     if (stream) cudaStreamSynchronize(stream);
     if (uploadStream) cudaStreamSynchronize(uploadStream);
+    hostCopy.reset();
     cudaMemPool_t pool = nullptr;
     if (device >= 0 && cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
     errWord.release();

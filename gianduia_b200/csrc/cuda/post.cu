@@ -15,6 +15,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "hostcopy.h"
 #include "runtime.h"
 
 namespace gnd {
@@ -321,11 +322,11 @@ gnd_status gnd_gpu_post(gnd_gpu_ctx* ctxh, const float* rgb, int32_t width, int3
         std::lock_guard<FairMutex> lk(c->mu);
         const size_t n = (size_t)width * height;
         PoolBuf din(n * 12, c->stream), dhdr(hdr ? n * 12 : 0, c->stream), d8(rgb8 ? n * 3 : 0, c->stream);
-        GND_CUDA(cudaMemcpyAsync(din.ptr, rgb, n * 12, cudaMemcpyHostToDevice, c->stream));
+        c->copies().in(din.ptr, rgb, n * 12, c->stream);
         postDevice(din.as<float>(), width, height, params, hdr ? dhdr.as<float>() : nullptr, rgb8 ? d8.as<uint8_t>() : nullptr,
                    c->stream);
-        if (hdr) GND_CUDA(cudaMemcpyAsync(hdr, dhdr.ptr, n * 12, cudaMemcpyDeviceToHost, c->stream));
-        if (rgb8) GND_CUDA(cudaMemcpyAsync(rgb8, d8.ptr, n * 3, cudaMemcpyDeviceToHost, c->stream));
+        if (hdr) c->copies().out(hdr, dhdr.ptr, n * 12, c->stream);
+        if (rgb8) c->copies().out(rgb8, d8.ptr, n * 3, c->stream);
         GND_CUDA(cudaStreamSynchronize(c->stream));
     });
 }

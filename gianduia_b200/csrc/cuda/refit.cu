@@ -11,6 +11,7 @@
 #include <cstring>
 #include <vector>
 
+#include "hostcopy.h"
 #include "runtime.h"
 
 namespace gnd {
@@ -49,6 +50,13 @@ __global__ void kRefitTris(const float* __restrict__ pos, int64_t n, const uint3
         t.v1x = p[3]; t.v1y = p[4]; t.v1z = p[5];
         t.v2x = p[6]; t.v2y = p[7]; t.v2z = p[8];
     }
+}
+
+// *bad = 1 when a value is NaN or infinite
+__global__ void kFinite(const float* __restrict__ v, int64_t n, uint32_t* bad) {
+    bool b = false;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) b = b || !isfinite(v[i]);
+    if (__any_sync(0xffffffffu, b) && (threadIdx.x & 31) == 0) *bad = 1u;
 }
 
 // One breadth-first step: the inner children of the nodes in `cur` are appended to `next`.
@@ -169,8 +177,6 @@ gnd_status gnd_gpu_scene_refit_mesh(gnd_gpu_ctx* ctxh, gnd_scene_id id, int32_t 
     return guarded([&]() {
         Context* c = ctxOf(ctxh);
         if (!positions && num_tris > 0) throw Error(GND_ERR_INVALID, "refit: null positions");
-        for (int64_t i = 0; i < 9 * num_tris; ++i)
-            if (!std::isfinite(positions[i])) throw Error(GND_ERR_INVALID, "refit: positions must be finite");
         c->bind();
         std::lock_guard<FairMutex> lk(c->mu);
         DeviceScene& ds = c->scene(id);
@@ -208,7 +214,17 @@ gnd_status gnd_gpu_scene_refit_mesh(gnd_gpu_ctx* ctxh, gnd_scene_id id, int32_t 
         const RefitTopo* tlas = v.tlasRoot != kEmpty ? &refitTopology(c, ds, v.tlasRoot) : nullptr;
         PoolBuf pos((size_t)num_tris * 9 * sizeof(float), c->stream);
         PoolBuf inst((size_t)std::max(ds.numInstances, 1) * sizeof(Box), c->stream);
-        GND_CUDA(cudaMemcpyAsync(pos.ptr, positions, pos.bytes, cudaMemcpyHostToDevice, c->stream));
+        c->copies().in(pos.ptr, positions, pos.bytes, c->stream);
+        // non-finite positions are refused before anything is changed (checked on the device:
+        // a host loop over 2.7M floats took 0.9 ms of a 2.3 ms call)
+        PoolBuf bad(16, c->stream);
+        uint32_t nonFinite = 0;
+        GND_CUDA(cudaMemsetAsync(bad.ptr, 0, 16, c->stream));
+        kFinite<<<gridFor(9 * num_tris, c->numSMs), 256, 0, c->stream>>>(pos.as<float>(), 9 * num_tris, bad.as<uint32_t>());
+        GND_CUDA(cudaGetLastError());
+        GND_CUDA(cudaMemcpyAsync(&nonFinite, bad.ptr, 4, cudaMemcpyDeviceToHost, c->stream));
+        GND_CUDA(cudaStreamSynchronize(c->stream));
+        if (nonFinite) throw Error(GND_ERR_INVALID, "refit: positions must be finite");
         // timing events, destroyed on every exit (a failing launch throws)
         struct Events {
             cudaEvent_t e[2] = {nullptr, nullptr};

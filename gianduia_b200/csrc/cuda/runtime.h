@@ -198,6 +198,7 @@ private:
 
 class Wavefront;
 class Server;
+class HostCopy;
 
 struct Context {
     int device = 0;
@@ -241,6 +242,8 @@ struct Context {
         uint32_t k = fetchNext++ % kFetchRing;
         return fetchRing.as<uint32_t>() + k;
     }
+    std::unique_ptr<HostCopy> hostCopy;   // staged copies of callers' pageable memory; used with mu held
+    HostCopy& copies();
     std::unique_ptr<Wavefront> wave;
     volatile bool cancel = false;
     // serving: HBM admission budget (0 = the device's free memory), queued or running
@@ -256,6 +259,7 @@ struct Context {
     std::map<uint64_t, int> sceneUse;
     std::mutex serverMu;
     std::unique_ptr<Server> server;
+    Context();
     ~Context();
     DeviceScene& scene(uint64_t id) {
         auto it = scenes.find(id);

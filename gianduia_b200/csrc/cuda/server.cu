@@ -3,6 +3,8 @@
 // runs a few engine iterations, reads every job's hand-out and retired counts, and
 // resolves the film of each job whose samples have all retired.
 #include <algorithm>
+#include <cstring>
+#include <new>
 
 #include "server.h"
 #include "wavefront.h"
@@ -11,6 +13,7 @@ namespace gnd {
 
 Server::Server(Context* c) : c_(c), t0_(std::chrono::steady_clock::now()) {
     thread_ = std::thread([this]() { loop(); });
+    finisher_ = std::thread([this]() { finishLoop(); });
 }
 
 Server::~Server() {
@@ -20,6 +23,16 @@ Server::~Server() {
     }
     workCv_.notify_all();
     if (thread_.joinable()) thread_.join();
+    {
+        std::lock_guard<std::mutex> lk(m_);
+        finishStop_ = true;   // films already queued are still delivered
+    }
+    finishCv_.notify_all();
+    if (finisher_.joinable()) finisher_.join();
+    for (Stage& s : stages_) {
+        if (s.host) cudaFreeHost(s.host);
+        if (s.copied) cudaEventDestroy(s.copied);
+    }
     // jobs still admitted are dropped with the engine; wake any waiter
     std::lock_guard<std::mutex> lk(m_);
     for (auto& kv : jobs_) {
@@ -41,6 +54,7 @@ uint64_t Server::bytesInUseLocked() const {
     uint64_t b = 0;
     for (const auto& kv : c_->scenes) b += kv.second->bytes;
     if (c_->wave) b += c_->wave->poolBytes() + c_->wave->jobBytes();
+    for (const Stage& s : stages_) b += s.dev.bytes;
     return b;
 }
 
@@ -128,10 +142,13 @@ gnd_status Server::wait(gnd_job_id id, float* film, gnd_job_status* st, int64_t 
         return GND_ERR_TIMEOUT;
     }
     fillStatus(*j, st);
-    if (film && !j->film.empty()) std::copy(j->film.begin(), j->film.end(), film);
+    const std::unique_ptr<float[]> done = std::move(j->film);
+    const size_t n = (size_t)j->W * j->H * 7;
     gnd_status s = j->state == GND_JOB_DONE ? GND_OK : (j->state == GND_JOB_CANCELLED ? GND_ERR_CANCELLED : j->status);
     if (s != GND_OK) err = j->state == GND_JOB_CANCELLED ? "job cancelled" : j->error;
     jobs_.erase(it);
+    lk.unlock();   // the serving threads do not wait for the caller's copy
+    if (film && done) std::memcpy(film, done.get(), n * sizeof(float));
     return s;
 }
 
@@ -143,21 +160,94 @@ void Server::cancel(gnd_job_id id) {
     workCv_.notify_all();
 }
 
-// Called with the context mutex held. Resolves the film (done or cancelled) and frees
-// the engine's job entry.
+Server::Stage& Server::freeStage(size_t bytes) {
+    Stage* s = nullptr;
+    {
+        std::unique_lock<std::mutex> lk(m_);
+        stageCv_.wait(lk, [&]() {
+            for (Stage& k : stages_)
+                if (!k.busy && (!s || k.bytes >= bytes)) s = &k;   // one that is large enough, if any
+            return s != nullptr;
+        });
+        s->busy = true;
+    }
+    try {
+        if (!s->copied) GND_CUDA(cudaEventCreateWithFlags(&s->copied, cudaEventDisableTiming));
+        if (s->bytes < bytes) {
+            if (s->host) cudaFreeHost(s->host);
+            s->host = nullptr;
+            s->bytes = 0;
+            s->dev.alloc(bytes);
+            GND_CUDA(cudaMallocHost(&s->host, bytes));
+            s->bytes = bytes;
+        }
+    } catch (...) {
+        std::lock_guard<std::mutex> lk(m_);
+        s->busy = false;
+        throw;
+    }
+    return *s;
+}
+
+// Called with the context mutex held. Queues the film's resolve and copy (done or
+// cancelled) and frees the engine's job entry; the rounds go on meanwhile. (The serving
+// thread used to wait for the copy and move the film itself, with the GPU idle: 10% of a
+// burst of twelve requests.)
 void Server::finishJob(ServeJob* j, int state) {
     Wavefront& wf = *c_->wave;
-    std::vector<float> film((size_t)j->W * j->H * 7);
-    wf.resolve(j->slot, film.data());
-    wf.drop(j->slot);
+    Stage& s = freeStage((size_t)j->W * j->H * 7 * sizeof(float));
+    try {
+        wf.resolveAsync(j->slot, s.dev.as<float>(), s.host);
+        GND_CUDA(cudaEventRecord(s.copied, c_->stream));
+        wf.drop(j->slot);
+    } catch (...) {
+        std::lock_guard<std::mutex> lk(m_);
+        s.busy = false;
+        throw;
+    }
     if (--c_->sceneUse[j->scene] <= 0) c_->sceneUse.erase(j->scene);
     std::lock_guard<std::mutex> lk(m_);
-    j->film.swap(film);
-    j->state = state;
-    j->tDone = nowMs();
     j->slot = -1;
     running_.erase(std::find(running_.begin(), running_.end(), j));
-    doneCv_.notify_all();
+    finished_.push_back(Finished{j, &s, state});
+    finishCv_.notify_one();
+}
+
+void Server::finishLoop() {
+    cudaSetDevice(c_->device);
+    std::unique_lock<std::mutex> lk(m_);
+    for (;;) {
+        finishCv_.wait(lk, [&]() { return finishStop_ || !finished_.empty(); });
+        if (finished_.empty()) return;
+        const Finished f = finished_.front();
+        finished_.pop_front();
+        lk.unlock();
+        const size_t n = (size_t)f.job->W * f.job->H * 7;
+        std::unique_ptr<float[]> film;
+        int state = f.state;
+        std::string why;
+        const cudaError_t e = cudaEventSynchronize(f.stage->copied);
+        if (e == cudaSuccess) {
+            film.reset(new (std::nothrow) float[n]);
+            if (film) std::memcpy(film.get(), f.stage->host, n * sizeof(float));
+            else why = "host allocation failed";
+        } else {
+            why = std::string("film copy: ") + cudaGetErrorString(e);
+        }
+        lk.lock();
+        ServeJob& j = *f.job;
+        f.stage->busy = false;
+        stageCv_.notify_all();
+        if (!film) {
+            state = GND_JOB_FAILED;
+            j.status = e == cudaSuccess ? GND_ERR_OOM : GND_ERR_CUDA;
+            j.error = why;
+        }
+        j.film = std::move(film);
+        j.state = state;
+        j.tDone = nowMs();
+        doneCv_.notify_all();
+    }
 }
 
 // Called with the context mutex held: every running job fails with `why`.

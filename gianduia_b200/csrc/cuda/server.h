@@ -32,7 +32,7 @@ struct ServeJob {
     int64_t firstRound = 0;          // first engine round whose counters include the job
     int64_t stopRound = -1;          // first round queued after its hand-out was stopped
     double tSubmit = 0, tAdmit = 0, tDone = 0;
-    std::vector<float> film;         // H x W x 7 once finished
+    std::unique_ptr<float[]> film;   // H x W x 7 once finished
     gnd_status status = GND_OK;
     std::string error;
 };
@@ -58,6 +58,29 @@ private:
     void fillStatus(const ServeJob& j, gnd_job_status* st) const;
     double nowMs() const;
     bool fitsLocked(const ServeJob& j) const;                // caller holds the context mutex
+    // Finished films leave beside the rounds: the serving thread queues the film's resolve and
+    // its copy into a pinned stage and goes on; the finishing thread waits for the copy, moves
+    // the film to the job and reports it.
+    struct Stage {
+        DevBuf dev;
+        float* host = nullptr;
+        size_t bytes = 0;
+        cudaEvent_t copied = nullptr;
+        bool busy = false;           // guarded by m_
+    };
+    struct Finished {
+        ServeJob* job;
+        Stage* stage;
+        int state;
+    };
+    static constexpr int kStages = 4;
+    Stage stages_[kStages];
+    Stage& freeStage(size_t bytes);                          // waits for one; caller holds the context mutex
+    void finishLoop();
+    std::thread finisher_;
+    std::condition_variable finishCv_, stageCv_;             // with m_
+    std::deque<Finished> finished_;
+    bool finishStop_ = false;
     void finishJob(ServeJob* j, int state);
     void failRunning(const std::string& why, gnd_status code);
     void drainPipeline();

@@ -3,6 +3,7 @@
 #include <mutex>
 #include <string>
 
+#include "hostcopy.h"
 #include "raysort.cuh"
 #include "runtime.h"
 #include "traverse.cuh"
@@ -175,8 +176,8 @@ void launchTrace(Context* c, DeviceScene& ds, const gnd_ray* dr, int64_t n, gnd_
     c->counters.trace_batches += 1;
 }
 
-// Host-buffer variant: copies in, traces, copies out (pinned staging is the caller's
-// concern; pageable memory works, at lower copy bandwidth).
+// Host-buffer variant: copies in, traces, copies out (pageable memory goes through the
+// context's staging).
 void traceHost(gnd_gpu_ctx* ctxh, gnd_scene_id id, const gnd_ray* rays, int64_t n, gnd_hit* hits, uint8_t* occ) {
     Context* c = ctxOf(ctxh);
     if (n < 0 || (n > 0 && (!rays || (!hits && !occ)))) throw Error(GND_ERR_INVALID, "bad ray batch arguments");
@@ -187,11 +188,10 @@ void traceHost(gnd_gpu_ctx* ctxh, gnd_scene_id id, const gnd_ray* rays, int64_t 
     size_t outBytes = hits ? sizeof(gnd_hit) * (size_t)n : (size_t)n;
     c->rayScratch.ensure(sizeof(gnd_ray) * (size_t)n);
     c->hitScratch.ensure(outBytes);
-    GND_CUDA(cudaMemcpyAsync(c->rayScratch.ptr, rays, sizeof(gnd_ray) * (size_t)n, cudaMemcpyHostToDevice, c->stream));
+    c->copies().in(c->rayScratch.ptr, rays, sizeof(gnd_ray) * (size_t)n, c->stream);
     launchTrace(c, ds, c->rayScratch.as<gnd_ray>(), n, hits ? c->hitScratch.as<gnd_hit>() : nullptr,
                 hits ? nullptr : c->hitScratch.as<uint8_t>(), nullptr, nullptr, c->stream);
-    GND_CUDA(cudaMemcpyAsync(hits ? (void*)hits : (void*)occ, c->hitScratch.ptr, outBytes, cudaMemcpyDeviceToHost, c->stream));
-    GND_CUDA(cudaStreamSynchronize(c->stream));
+    c->copies().out(hits ? (void*)hits : (void*)occ, c->hitScratch.ptr, outBytes, c->stream);
     c->checkKernelErrors("trace");
 }
 }  // namespace

@@ -20,6 +20,7 @@
 #include <chrono>
 #include <cstring>
 
+#include "hostcopy.h"
 #include "raysort.cuh"
 #include "shading.cuh"
 #include "textures.cuh"
@@ -816,6 +817,15 @@ __device__ __forceinline__ void beginIteration(uint32_t* cnt, uint32_t in, uint3
     for (int k = 0; k < kShadeClasses; ++k) cnt[kQClass0 + k] = 0;
     cnt[kQWork] = work ? 1u : 0u;
     cnt[kQFreeOut] = work ? 0u : idle;
+}
+
+// The active job list, by value: no staging to wait for.
+struct ActiveIds {
+    uint32_t n, id[kMaxJobs];
+};
+__global__ void kSetActive(ActiveIds a, uint32_t* active, uint32_t* cnt) {
+    if (threadIdx.x < a.n) active[threadIdx.x] = a.id[threadIdx.x];
+    if (threadIdx.x == 0) cnt[kQActive] = a.n;
 }
 
 // Start of a round of at most `pairs` iteration pairs: the host may have admitted, released
@@ -1893,11 +1903,12 @@ void Wavefront::syncActive() {
     std::sort(ids, ids + n, [&](uint32_t a, uint32_t b) {
         return jobs_[a].prio != jobs_[b].prio ? jobs_[a].prio < jobs_[b].prio : jobs_[a].seq < jobs_[b].seq;
     });
-    cudaStream_t st = ctx_->stream;
-    if (n) GND_CUDA(cudaMemcpyAsync(active_.ptr, ids, n * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-    GND_CUDA(cudaMemcpyAsync(counters_.as<uint32_t>() + kQActive, &n, sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-    // the staging arrays are on the stack: wait for the copies before returning
-    GND_CUDA(cudaStreamSynchronize(st));
+    ActiveIds a;
+    a.n = n;
+    std::copy(ids, ids + n, a.id);
+    kSetActive<<<1, kMaxJobs, 0, ctx_->stream>>>(a, active_.as<uint32_t>(), counters_.as<uint32_t>());
+    ++launches_;
+    GND_CUDA(cudaGetLastError());
     activeDirty_ = false;
 }
 
@@ -2065,20 +2076,20 @@ const float* Wavefront::resolvePinned(int j) {
         GND_CUDA(cudaMallocHost(&pinnedFilm_, bytes));
         pinnedFilmBytes_ = bytes;
     }
-    cudaStream_t st = ctx_->stream;
-    int grid = (int)std::min<size_t>((npix + 255) / 256, (size_t)ctx_->numSMs * 8);
-    kFilmResolve<<<std::max(grid, 1), 256, 0, st>>>(hj.filmSum.as<unsigned long long>(), hj.filmSq.as<float>(),
-                                                    filmOut_.as<float>(), npix);
-    ++launches_;
-    GND_CUDA(cudaGetLastError());
-    GND_CUDA(cudaMemcpyAsync(pinnedFilm_, filmOut_.ptr, bytes, cudaMemcpyDeviceToHost, st));
-    GND_CUDA(cudaStreamSynchronize(st));
+    resolveAsync(j, filmOut_.as<float>(), pinnedFilm_);
+    GND_CUDA(cudaStreamSynchronize(ctx_->stream));
     return pinnedFilm_;
 }
 
-void Wavefront::resolve(int j, float* filmHost) {
-    const float* f = resolvePinned(j);
-    std::memcpy(filmHost, f, (size_t)jobs_[j].dev.W * jobs_[j].dev.H * 7 * sizeof(float));
+void Wavefront::resolveAsync(int j, float* dev, float* host) {
+    const HostJob& hj = jobs_[j];
+    const size_t npix = (size_t)hj.dev.W * hj.dev.H;
+    cudaStream_t st = ctx_->stream;
+    int grid = (int)std::min<size_t>((npix + 255) / 256, (size_t)ctx_->numSMs * 8);
+    kFilmResolve<<<std::max(grid, 1), 256, 0, st>>>(hj.filmSum.as<unsigned long long>(), hj.filmSq.as<float>(), dev, npix);
+    ++launches_;
+    GND_CUDA(cudaGetLastError());
+    GND_CUDA(cudaMemcpyAsync(host, dev, npix * 7 * sizeof(float), cudaMemcpyDeviceToHost, st));
 }
 
 void Wavefront::finish(int j, float* filmHost) {
@@ -2086,7 +2097,12 @@ void Wavefront::finish(int j, float* filmHost) {
     const size_t n = (size_t)hj.dev.W * hj.dev.H * 7;
     if (filmHost) {
         const float* f = resolvePinned(j);
-        for (size_t q = 0; q < n; ++q) filmHost[q] += f[q];
+        auto add = [&](size_t b, size_t e) {
+            for (size_t q = b; q < e; ++q) filmHost[q] += f[q];
+        };
+        // below 4 MB one thread is done before the others are awake
+        if (n * sizeof(float) < size_t(4) << 20) add(0, n);
+        else ctx_->copies().parallel(n, size_t(1) << 18, add);
     }
     drop(j);
 }

@@ -132,7 +132,8 @@ public:
     void finish(int job, float* filmHost);            // adds the film to filmHost, frees the job
     // adds the job's fixed-point sums into sum (H x W x 4) and sq (H x W x 3), frees the job
     void finishFixed(int job, uint64_t* sum, float* sq);
-    void resolve(int job, float* filmHost);           // writes the film (H x W x 7 floats) to filmHost
+    // Queues the film's resolve into `dev` and its copy to pinned `host` (H x W x 7 floats each).
+    void resolveAsync(int job, float* dev, float* host);
     // The job's film resolved into pinned host memory (valid until the next call).
     const float* resolvePinned(int job);
     void stop(int job);                               // hands out no further work items of the job

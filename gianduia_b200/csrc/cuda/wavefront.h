@@ -103,6 +103,7 @@ struct HostJob {
 // graph launch whose loop over iteration pairs runs on the device (conditional node) and
 // ends with the last path, so neither the host nor empty iterations stand between them.
 struct KParams;
+struct Fork;
 
 class Wavefront {
 public:
@@ -205,6 +206,7 @@ private:
     bool motion_ = false;   // an admitted job's scene has animated instances (MOTION traversal)
     bool ext_ = false;      // an admitted job's scene uses the EXT features (SceneView::ext)
     bool textured_ = false; // an admitted job's scene has texture trees
+    std::unique_ptr<Fork> fork_;   // side streams of the shade classes
     std::vector<GraphEntry> graphs_;
     Tune tune_;
     Context* ctx_;

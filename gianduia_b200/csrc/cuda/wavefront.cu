@@ -2310,7 +2310,10 @@ cudaGraphExec_t Wavefront::roundGraph(const KParams& kp, int par, int mix, bool 
         if (g.par == par && g.mix == mix && g.pairs == pairs && g.classes == cls && g.hasNull == hasNull && g.fifo == fifo &&
             g.motion == motion_ && g.ext == ext_ && g.textured == textured_)
             return g.exec;
-    if (graphs_.size() >= 64) clearGraphs();   // served mixes of scenes come and go
+    if (graphs_.size() >= 64) {   // served mixes of scenes come and go
+        GND_CUDA(cudaStreamSynchronize(st));
+        clearGraphs();
+    }
     struct Guard {
         cudaGraph_t g = nullptr;
         ~Guard() {

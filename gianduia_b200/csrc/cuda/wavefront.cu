@@ -2002,10 +2002,11 @@ int Wavefront::admit(const DeviceScene& ds, int W, int H, int spp, int firstPass
     jd.workEnd = hj.released;
     jd.passItems = passItems;
     jd.total = hj.total;
-    // class 4 (every lobe): null-BSDF surfaces, and escaped paths that are still shaded
+    // class 4 (every lobe): surfaces without a BSDF -- the index material and, with it, every
+    // material type beyond it (SceneView::instClass) -- and escaped paths that are still shaded
     // (shadeClass, ExtendSrc::store)
-    uint32_t cls = ds.matTypes & 15u;
-    if (ds.hasNullMaterials || integrator == 1 || ds.view.env.emitter >= 0) cls |= 16u;
+    uint32_t cls = ds.matTypes & ((2u << kMatIndex) - 1u);
+    if (integrator == 1 || ds.view.env.emitter >= 0) cls |= 1u << kMatIndex;
     if (integrator == 1) cls |= 1u << kMediumClass;
     hj.classes = integrator == 1 ? cls << kClassesPerInt : cls;
     hj.used = true;

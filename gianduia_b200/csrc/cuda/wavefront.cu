@@ -21,6 +21,7 @@
 #include <cstring>
 
 #include "hostcopy.h"
+#include "progress.h"
 #include "raysort.cuh"
 #include "shading.cuh"
 #include "textures.cuh"
@@ -2472,6 +2473,7 @@ Wavefront::Result Wavefront::render(DeviceScene& ds, int W, int H, int spp, int 
             // iterations, one queued ahead of the one whose counters the host is reading
             const int kRoundIters = std::min(std::max(tune_.roundIters & ~1, 2), 64);
             int64_t k = 0, stopAt = -1;
+            RoundProgress progress;
             enqueueRound(kRoundIters, mix, ds.hasNullMaterials, profile, res, 0);
             for (;;) {
                 enqueueRound(kRoundIters, mix, ds.hasNullMaterials, profile, res, (int)((k + 1) & 1));
@@ -2481,6 +2483,8 @@ Wavefront::Result Wavefront::render(DeviceScene& ds, int W, int H, int spp, int 
                 if (r >= total && inflight == 0) break;
                 // after a cancel, only rounds queued after the stop show the final state
                 if (cancelled && k > stopAt && inflight == 0) break;
+                if (!cancelled && progress.stuck(sn.iterations, r, inflight, total))
+                    throw Error(GND_ERR_DEVICE_CHECK, "paths lost: " + std::to_string(total - r) + " samples cannot be finished");
                 if (c->cancel && !cancelled) {
                     if (batched) stop(j);   // queued behind round k + 1
                     else stopPasses(j);     // the passes released so far are finished

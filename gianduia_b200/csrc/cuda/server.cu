@@ -62,15 +62,30 @@ size_t Server::poolSlots() const {
     return size_t(1) << std::min(std::max(c_->serveTune.poolLog2, 16), 26);
 }
 
-bool Server::fitsLocked(const ServeJob& j) const {
-    const size_t slots = poolSlots();
-    const uint64_t pool = c_->wave && c_->wave->capacity() >= slots ? 0 : Wavefront::slotBytes() * slots;
-    const uint64_t staging = (uint64_t)j.W * j.H * 7 * sizeof(float);
-    const uint64_t need = j.filmBytes + staging + pool;
-    if (c_->hbmBudget) return bytesInUseLocked() + need <= c_->hbmBudget;
+static uint64_t stagingBytes(const ServeJob& j) { return (uint64_t)j.W * j.H * 7 * sizeof(float); }
+
+// A running job's film leaves through one stage; several only let films leave side by side. So
+// room is kept for one stage of the largest running film, and whatever else the stages hold
+// goes when a job waits for memory.
+uint64_t Server::stageGrowth(uint64_t bytes) const {
+    uint64_t largest = 0;
+    for (const Stage& s : stages_) largest = std::max<uint64_t>(largest, s.dev.bytes);
+    for (const ServeJob* j : running_) bytes = std::max(bytes, stagingBytes(*j));
+    return bytes > largest ? bytes - largest : 0;
+}
+
+int64_t Server::filmGrowth(const ServeJob& j, int ahead) const {
+    return (int64_t)j.filmBytes - (c_->wave ? (int64_t)c_->wave->idleFilmBytes(ahead) : 0);
+}
+
+bool Server::fitsLocked(const ServeJob& j, const Ahead& a) const {
+    const size_t slots = poolSlots(), cap = c_->wave ? c_->wave->capacity() : 0;
+    const int64_t pool = cap >= slots ? 0 : (int64_t)(Wavefront::slotBytes() * (slots - cap));
+    const int64_t need = filmGrowth(j, a.jobs) + a.filmBytes + (int64_t)stageGrowth(std::max(a.staging, stagingBytes(j))) + pool;
+    if (c_->hbmBudget) return (int64_t)bytesInUseLocked() + need <= (int64_t)c_->hbmBudget;
     size_t freeB = 0, totalB = 0;
     if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess) return false;
-    return need + (uint64_t(256) << 20) <= freeB;
+    return need + (int64_t(256) << 20) <= (int64_t)freeB;
 }
 
 gnd_job_id Server::submit(const gnd_job_desc& d) {
@@ -160,33 +175,69 @@ void Server::cancel(gnd_job_id id) {
     workCv_.notify_all();
 }
 
+void Server::dropStage(Stage& s) {
+    s.dev.release();
+    if (s.host) cudaFreeHost(s.host);
+    s.host = nullptr;
+    s.bytes = 0;
+}
+
+void Server::trimStagesLocked(uint64_t bytes, bool larger) {
+    Stage* keep = nullptr;
+    for (Stage& s : stages_)
+        if ((s.bytes == bytes || (larger && s.bytes > bytes)) && (!keep || s.bytes < keep->bytes)) keep = &s;
+    for (Stage& s : stages_)
+        if (!s.busy && &s != keep) dropStage(s);
+}
+
+// The smallest idle stage that is large enough, else the largest one grown to the size. Under
+// a budget a stage grows only within it: otherwise the stages in use are waited for and
+// the idle ones freed first (fitsLocked kept room for one stage of this size). The same when
+// there is no memory for it.
 Server::Stage& Server::freeStage(size_t bytes) {
     Stage* s = nullptr;
-    {
-        std::unique_lock<std::mutex> lk(m_);
-        stageCv_.wait(lk, [&]() {
-            for (Stage& k : stages_)
-                if (!k.busy && (!s || k.bytes >= bytes)) s = &k;   // one that is large enough, if any
-            return s != nullptr;
-        });
-        s->busy = true;
-    }
-    try {
-        if (!s->copied) GND_CUDA(cudaEventCreateWithFlags(&s->copied, cudaEventDisableTiming));
-        if (s->bytes < bytes) {
-            if (s->host) cudaFreeHost(s->host);
-            s->host = nullptr;
-            s->bytes = 0;
-            s->dev.alloc(bytes);
-            GND_CUDA(cudaMallocHost(&s->host, bytes));
-            s->bytes = bytes;
+    bool alone = false;   // wait until every stage is idle, keep only the one taken
+    for (;;) {
+        {
+            std::unique_lock<std::mutex> lk(m_);
+            for (;;) {
+                Stage *fit = nullptr, *largest = nullptr;
+                bool busy = false;
+                for (Stage& k : stages_) {
+                    busy = busy || k.busy;
+                    if (k.busy) continue;
+                    if (k.bytes >= bytes && (!fit || k.bytes < fit->bytes)) fit = &k;
+                    if (!largest || k.bytes > largest->bytes) largest = &k;
+                }
+                s = fit ? fit : largest;
+                if (fit) break;
+                if (s && !alone && (!c_->hbmBudget || bytesInUseLocked() - s->dev.bytes + bytes <= c_->hbmBudget)) break;
+                if (s && !busy) {
+                    for (Stage& k : stages_) dropStage(k);
+                    break;
+                }
+                stageCv_.wait(lk);
+            }
+            s->busy = true;
         }
-    } catch (...) {
-        std::lock_guard<std::mutex> lk(m_);
-        s->busy = false;
-        throw;
+        try {
+            if (!s->copied) GND_CUDA(cudaEventCreateWithFlags(&s->copied, cudaEventDisableTiming));
+            if (s->bytes < bytes) {
+                dropStage(*s);
+                s->dev.alloc(bytes);
+                GND_CUDA(cudaMallocHost(&s->host, bytes));
+                s->bytes = bytes;
+            }
+            return *s;
+        } catch (const Error& e) {
+            std::lock_guard<std::mutex> lk(m_);
+            dropStage(*s);
+            s->busy = false;
+            if (alone || e.code != GND_ERR_OOM) throw;
+            cudaGetLastError();
+        }
+        alone = true;
     }
-    return *s;
 }
 
 // Called with the context mutex held. Queues the film's resolve and copy (done or
@@ -298,6 +349,7 @@ void Server::loop() {
             // admission, first come first served
             std::vector<ServeJob*> admit;
             {
+                Ahead ahead;
                 std::lock_guard<std::mutex> lk(m_);
                 while (!queue_.empty() && running_.size() + admit.size() < (size_t)kMaxJobs) {
                     ServeJob* j = jobs_.at(queue_.front()).get();
@@ -309,8 +361,19 @@ void Server::loop() {
                         doneCv_.notify_all();
                         continue;
                     }
-                    if (!fitsLocked(*j)) break;
+                    if (!fitsLocked(*j, ahead)) {
+                        // with what earlier jobs and renders left idle freed, a job that was
+                        // accepted fits at the latest when nothing else runs
+                        uint64_t largest = std::max(ahead.staging, stagingBytes(*j));
+                        for (const ServeJob* r : running_) largest = std::max(largest, stagingBytes(*r));
+                        trimStagesLocked(largest, true);
+                        if (admit.empty()) wf.releaseIdle(poolSlots());
+                        if (!fitsLocked(*j, ahead)) trimStagesLocked(largest, false);
+                        if (!fitsLocked(*j, ahead)) break;
+                    }
                     queue_.pop_front();
+                    ahead.filmBytes += filmGrowth(*j, ahead.jobs++);
+                    ahead.staging = std::max(ahead.staging, stagingBytes(*j));
                     admit.push_back(j);
                 }
             }

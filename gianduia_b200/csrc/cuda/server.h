@@ -57,7 +57,16 @@ private:
     void loop();
     void fillStatus(const ServeJob& j, gnd_job_status* st) const;
     double nowMs() const;
-    bool fitsLocked(const ServeJob& j) const;                // caller holds the context mutex
+    // Whether the job fits beside the running ones and those collected for admission before it
+    // (their number, the film bytes they add, their largest film); caller holds the context
+    // mutex and m_.
+    struct Ahead {
+        int jobs = 0;
+        int64_t filmBytes = 0;
+        uint64_t staging = 0;
+    };
+    bool fitsLocked(const ServeJob& j, const Ahead& a) const;
+    int64_t filmGrowth(const ServeJob& j, int ahead) const;  // film bytes that admitting the job adds
     // Finished films leave beside the rounds: the serving thread queues the film's resolve and
     // its copy into a pinned stage and goes on; the finishing thread waits for the copy, moves
     // the film to the job and reports it.
@@ -74,8 +83,11 @@ private:
         int state;
     };
     static constexpr int kStages = 4;
-    Stage stages_[kStages];
+    Stage stages_[kStages];                                  // memory changed with the context mutex held
     Stage& freeStage(size_t bytes);                          // waits for one; caller holds the context mutex
+    static void dropStage(Stage& s);                         // frees its memory
+    uint64_t stageGrowth(uint64_t bytes) const;              // what the stages lack of one for every running film
+    void trimStagesLocked(uint64_t bytes, bool larger);      // frees idle stages but one of that size (or larger)
     void finishLoop();
     std::thread finisher_;
     std::condition_variable finishCv_, stageCv_;             // with m_

@@ -1866,6 +1866,30 @@ uint64_t Wavefront::poolBytes() const {
         if (!j.used) b += j.filmSum.bytes + j.filmSq.bytes;
     return b;
 }
+uint64_t Wavefront::idleFilmBytes(int k) const {
+    for (const HostJob& j : jobs_)
+        if (!j.used && k-- == 0) return j.filmSum.bytes + j.filmSq.bytes;
+    return 0;
+}
+void Wavefront::releaseIdle(size_t slots) {
+    const bool pool = !busy() && cap_ > slots;
+    bool films = filmOut_.bytes > 0;
+    for (const HostJob& j : jobs_) films = films || (!j.used && j.filmSum.bytes + j.filmSq.bytes > 0);
+    if (!pool && !films) return;
+    GND_CUDA(cudaStreamSynchronize(ctx_->stream));   // queued resolves and rounds still use them
+    for (HostJob& j : jobs_) {
+        if (j.used) continue;
+        j.filmSum.release();
+        j.filmSq.release();
+    }
+    filmOut_.release();
+    if (!pool) return;
+    clearGraphs();
+    for (DevBuf* b : {&paths_, &times_, &hits_, &listA_, &listB_, &freeA_, &freeB_, &shadow_, &done_, &classes_, &rayKeys_, &raySorted_})
+        b->release();
+    cap_ = 0;
+}
+
 Wavefront::~Wavefront() {
     for (cudaEvent_t e : evPool_) cudaEventDestroy(e);
     if (evStart_) cudaEventDestroy(evStart_);

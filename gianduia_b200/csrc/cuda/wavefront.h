@@ -181,6 +181,10 @@ public:
                2 * sizeof(uint32_t);   // ray keys and the reordered list
     }
     uint64_t poolBytes() const;   // path pool + film staging + film buffers kept for reuse
+    uint64_t idleFilmBytes(int k) const;   // film buffers kept in the job slot that the k-th admission from now takes
+    // Frees what no admitted job uses: film buffers kept for reuse, render()'s film staging and,
+    // with no job admitted, a pool of more than `slots` path slots.
+    void releaseIdle(size_t slots);
     HostJob& job(int j) { return jobs_[j]; }
     uint64_t jobBytes() const;
 

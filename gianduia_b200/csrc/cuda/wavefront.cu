@@ -1891,6 +1891,7 @@ void Wavefront::releaseIdle(size_t slots) {
 }
 
 Wavefront::~Wavefront() {
+    cudaStreamSynchronize(ctx_->stream);   // a round may be queued: it writes the snapshots
     for (cudaEvent_t e : evPool_) cudaEventDestroy(e);
     if (evStart_) cudaEventDestroy(evStart_);
     if (evEnd_) cudaEventDestroy(evEnd_);
@@ -2325,6 +2326,10 @@ int Wavefront::launchesPerIteration(int mix) const {
 }
 
 void Wavefront::clearGraphs() {
+    if (graphs_.empty()) return;
+    // A round may still be executing one of them: neither a finished job nor the pool's reset
+    // waits for the round queued ahead. (Errors are the next call's to report.)
+    cudaStreamSynchronize(ctx_->stream);
     for (GraphEntry& g : graphs_) cudaGraphExecDestroy(g.exec);
     graphs_.clear();
 }
@@ -2336,10 +2341,7 @@ cudaGraphExec_t Wavefront::roundGraph(const KParams& kp, int par, int mix, bool 
         if (g.par == par && g.mix == mix && g.pairs == pairs && g.classes == cls && g.hasNull == hasNull && g.fifo == fifo &&
             g.motion == motion_ && g.ext == ext_ && g.textured == textured_)
             return g.exec;
-    if (graphs_.size() >= 64) {   // served mixes of scenes come and go
-        GND_CUDA(cudaStreamSynchronize(st));
-        clearGraphs();
-    }
+    if (graphs_.size() >= 64) clearGraphs();   // served mixes of scenes come and go
     struct Guard {
         cudaGraph_t g = nullptr;
         ~Guard() {

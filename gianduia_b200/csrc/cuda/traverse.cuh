@@ -347,6 +347,13 @@ __device__ __forceinline__ void nodeKeysFast(const Node4* nd, const Trav& t, uin
     }
 }
 
+// The same direction bit for bit: 0 and -0 have reciprocals of opposite sign, and the exact slab
+// test tells them apart when the origin lies on a box plane.
+__device__ __forceinline__ bool sameDir(V3 a, V3 b) {
+    return ((__float_as_uint(a.x) ^ __float_as_uint(b.x)) | (__float_as_uint(a.y) ^ __float_as_uint(b.y)) |
+            (__float_as_uint(a.z) ^ __float_as_uint(b.z))) == 0u;
+}
+
 // Gives the lane reference `e` to work on: an inner node, or a leaf to hold.
 __device__ __forceinline__ void travTake(Trav& t, uint32_t e) {
     const bool leaf = isLeaf(e);
@@ -367,7 +374,7 @@ __device__ __forceinline__ void travPop(Trav& t, const Stack& st, const Src& src
         if (e.ref == kSentinel) {
             const V3 od = t.d;
             src.world(t.o, t.d, t.tmin);
-            if (!(od.x == t.d.x && od.y == t.d.y && od.z == t.d.z)) t.inv = v3(__frcp_rn(t.d.x), __frcp_rn(t.d.y), __frcp_rn(t.d.z));
+            if (!sameDir(od, t.d)) t.inv = v3(__frcp_rn(t.d.x), __frcp_rn(t.d.y), __frcp_rn(t.d.z));
             t.fast = t.wfast;
             t.curInst = -1;
             if constexpr (CULL) cull = cullKey(t);
@@ -476,7 +483,7 @@ __device__ __forceinline__ int travInstStep(Trav& t, const SceneView& s, Stack& 
         st.put(t.sp++, kSentinel, 0u);
         t.cur = root;
         // a translation keeps the direction, and with it the three reciprocals
-        if (!(ld.x == t.d.x && ld.y == t.d.y && ld.z == t.d.z)) t.inv = v3(__frcp_rn(ld.x), __frcp_rn(ld.y), __frcp_rn(ld.z));
+        if (!sameDir(ld, t.d)) t.inv = v3(__frcp_rn(ld.x), __frcp_rn(ld.y), __frcp_rn(ld.z));
         t.o = lo; t.d = ld;
         t.fast = t.wfast && slabFinite(s, lo, t.inv);
         t.tmin = kEpsilon;

@@ -114,9 +114,10 @@ void HostCopy::parallel(size_t n, size_t piece, const std::function<void(size_t,
 }
 
 void HostCopy::in(void* dst, const void* src, size_t bytes, cudaStream_t st) {
-    if (bytes <= kSmall || pinned(src)) {
+    const bool direct = pinned(src);
+    if (bytes <= kSmall || direct) {
         GND_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
-        if (bytes > kSmall) GND_CUDA(cudaStreamSynchronize(st));   // pinned: the bus still reads it
+        if (direct) GND_CUDA(cudaStreamSynchronize(st));   // the bus still reads it
         return;
     }
     for (size_t at = 0; at < bytes; at += kStage) {

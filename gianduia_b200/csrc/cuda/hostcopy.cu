@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <system_error>
 
 namespace gnd {
 
@@ -28,26 +29,34 @@ bool HostCopy::pinned(const void* p) {
     return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged;
 }
 
-// Room for `bytes` in the staging buffer, nothing still being read from it.
-void HostCopy::reserve(size_t bytes) {
+// Room for `bytes` in the staging buffer, nothing still being read from it. False when no
+// pinned memory can be had: the copy is then made plainly.
+bool HostCopy::reserve(size_t bytes) {
     if (!busy_) GND_CUDA(cudaEventCreateWithFlags(&busy_, cudaEventDisableTiming));
     if (pending_) {
         GND_CUDA(cudaEventSynchronize(busy_));
         pending_ = false;
     }
-    if (bytes <= stageBytes_) return;
+    if (bytes <= stageBytes_) return true;
     if (stage_) GND_CUDA(cudaFreeHost(stage_));
     stage_ = nullptr;
     stageBytes_ = 0;
     size_t n = kChunk * 4;
     while (n < bytes) n *= 2;
-    GND_CUDA(cudaMallocHost(&stage_, n));
-    stageBytes_ = n;
-    while (events_.size() < n / kChunk) {
-        cudaEvent_t e = nullptr;
-        GND_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        events_.push_back(e);
+    const cudaError_t e = cudaMallocHost(&stage_, n);
+    if (e != cudaSuccess) {
+        stage_ = nullptr;
+        cudaGetLastError();
+        if (e == cudaErrorMemoryAllocation) return false;
+        GND_CUDA(e);
     }
+    while (events_.size() < n / kChunk) {
+        cudaEvent_t ev = nullptr;
+        GND_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        events_.push_back(ev);
+    }
+    stageBytes_ = n;
+    return true;
 }
 
 void HostCopy::takeTasks() {
@@ -84,7 +93,11 @@ void HostCopy::run(int tasks, const std::function<void(int)>& f) {
     if (threads_.empty()) {
         const unsigned hw = std::thread::hardware_concurrency();
         const int n = std::min<int>(kWorkers, hw > 1 ? (int)hw - 1 : 0);
-        for (int k = 0; k < n; ++k) threads_.emplace_back([this]() { worker(); });
+        try {
+            for (int k = 0; k < n; ++k) threads_.emplace_back([this]() { worker(); });
+        } catch (const std::system_error&) {
+            // as many as there are: the calling thread takes the remaining tasks
+        }
     }
     {
         std::lock_guard<std::mutex> lk(m_);
@@ -122,7 +135,10 @@ void HostCopy::in(void* dst, const void* src, size_t bytes, cudaStream_t st) {
     }
     for (size_t at = 0; at < bytes; at += kStage) {
         const size_t n = std::min(kStage, bytes - at);
-        reserve(n);
+        if (!reserve(n)) {
+            GND_CUDA(cudaMemcpyAsync((char*)dst + at, (const char*)src + at, bytes - at, cudaMemcpyHostToDevice, st));
+            return;
+        }
         std::atomic<int> err{(int)cudaSuccess};
         run((int)((n + kChunk - 1) / kChunk), [&](int k) {
             const size_t o = (size_t)k * kChunk, m = std::min(kChunk, n - o);
@@ -144,7 +160,11 @@ void HostCopy::out(void* dst, const void* src, size_t bytes, cudaStream_t st) {
     }
     for (size_t at = 0; at < bytes; at += kStage) {
         const size_t n = std::min(kStage, bytes - at);
-        reserve(n);
+        if (!reserve(n)) {
+            GND_CUDA(cudaMemcpyAsync((char*)dst + at, (const char*)src + at, bytes - at, cudaMemcpyDeviceToHost, st));
+            GND_CUDA(cudaStreamSynchronize(st));
+            return;
+        }
         const int chunks = (int)((n + kChunk - 1) / kChunk);
         for (int k = 0; k < chunks; ++k) {
             const size_t o = (size_t)k * kChunk, m = std::min(kChunk, n - o);

@@ -34,7 +34,7 @@ public:
     void parallel(size_t n, size_t piece, const std::function<void(size_t, size_t)>& f);
 
 private:
-    void reserve(size_t bytes);
+    bool reserve(size_t bytes);
     void run(int tasks, const std::function<void(int)>& f);   // f(0) .. f(tasks - 1), all done on return
     void worker();
     static bool pinned(const void* p);

@@ -3,6 +3,10 @@
 // names the case; exit code 0 when it holds.
 #include "hostcopy.h"
 
+#include <dlfcn.h>
+#include <pthread.h>
+
+#include <cerrno>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -18,6 +22,8 @@ struct Range {
 std::mutex gMu;
 std::vector<Range> gRanges;                       // everything else is pageable
 std::vector<std::function<void()>> gQueue;        // the one stream
+bool gNoPinned = false;                           // pinned memory cannot be had
+int gThreads = -1;                                // threads that can still be started (-1: any number)
 
 cudaMemoryType typeOf(const void* p) {
     for (const Range& r : gRanges)
@@ -31,6 +37,12 @@ void drain() {
 }  // namespace
 
 extern "C" {
+int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), void* arg) {
+    if (gThreads == 0) return EAGAIN;
+    if (gThreads > 0) --gThreads;
+    using Create = int (*)(pthread_t*, const pthread_attr_t*, void* (*)(void*), void*);
+    return reinterpret_cast<Create>(dlsym(RTLD_NEXT, "pthread_create"))(t, a, f, arg);
+}
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind, cudaStream_t) {
     std::lock_guard<std::mutex> lk(gMu);
     const bool pageable = typeOf(dst) == cudaMemoryTypeUnregistered || typeOf(src) == cudaMemoryTypeUnregistered;
@@ -61,6 +73,7 @@ cudaError_t cudaEventDestroy(cudaEvent_t e) {
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaStreamSynchronize(nullptr); }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) {
+    if (gNoPinned) return cudaErrorMemoryAllocation;
     std::lock_guard<std::mutex> lk(gMu);
     *p = std::malloc(n);
     gRanges.push_back({(const char*)*p, n, cudaMemoryTypeHost});
@@ -123,5 +136,13 @@ int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "pageable") return roundTrip(cudaMemoryTypeUnregistered) ? 0 : 1;
     if (what == "pinned") return roundTrip(cudaMemoryTypeHost) ? 0 : 1;
+    if (what == "no-pinned-memory") {
+        gNoPinned = true;
+        return roundTrip(cudaMemoryTypeUnregistered) ? 0 : 1;
+    }
+    if (what == "no-threads" || what == "one-thread") {
+        gThreads = what == "one-thread" ? 1 : 0;
+        return roundTrip(cudaMemoryTypeUnregistered) ? 0 : 1;
+    }
     return 2;
 }

@@ -20,13 +20,13 @@ HostCopy::~HostCopy() {
     if (stage_) cudaFreeHost(stage_);
 }
 
-bool HostCopy::pinned(const void* p) {
+bool HostCopy::pageable(const void* p) {
     cudaPointerAttributes a{};
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return true;
     }
-    return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged;
+    return a.type == cudaMemoryTypeUnregistered;
 }
 
 // Room for `bytes` in the staging buffer, nothing still being read from it. False when no
@@ -127,7 +127,7 @@ void HostCopy::parallel(size_t n, size_t piece, const std::function<void(size_t,
 }
 
 void HostCopy::in(void* dst, const void* src, size_t bytes, cudaStream_t st) {
-    const bool direct = pinned(src);
+    const bool direct = !pageable(src);
     if (bytes <= kSmall || direct) {
         GND_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
         if (direct) GND_CUDA(cudaStreamSynchronize(st));   // the bus still reads it
@@ -153,7 +153,7 @@ void HostCopy::in(void* dst, const void* src, size_t bytes, cudaStream_t st) {
 }
 
 void HostCopy::out(void* dst, const void* src, size_t bytes, cudaStream_t st) {
-    if (bytes <= kSmall || pinned(dst)) {
+    if (bytes <= kSmall || !pageable(dst)) {
         GND_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st));
         GND_CUDA(cudaStreamSynchronize(st));
         return;

@@ -37,7 +37,8 @@ private:
     bool reserve(size_t bytes);
     void run(int tasks, const std::function<void(int)>& f);   // f(0) .. f(tasks - 1), all done on return
     void worker();
-    static bool pinned(const void* p);
+    // Memory that only the host can read; the rest (pinned, managed, device) is the runtime's to copy.
+    static bool pageable(const void* p);
 
     const int device_;
     char* stage_ = nullptr;

@@ -23,6 +23,7 @@ std::mutex gMu;
 std::vector<Range> gRanges;                       // everything else is pageable
 std::vector<std::function<void()>> gQueue;        // the one stream
 bool gNoPinned = false;                           // pinned memory cannot be had
+int gDirect = 0;                                  // copies between two ranges neither of which is pinned or pageable
 int gThreads = -1;                                // threads that can still be started (-1: any number)
 
 cudaMemoryType typeOf(const void* p) {
@@ -46,9 +47,8 @@ int pthread_create(pthread_t* t, const pthread_attr_t* a, void* (*f)(void*), voi
 cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind, cudaStream_t) {
     std::lock_guard<std::mutex> lk(gMu);
     const bool pageable = typeOf(dst) == cudaMemoryTypeUnregistered || typeOf(src) == cudaMemoryTypeUnregistered;
-    auto copy = [=]() {
-        std::memcpy(dst, src, n);
-    };
+    if (typeOf(dst) == cudaMemoryTypeDevice && typeOf(src) == cudaMemoryTypeDevice) ++gDirect;
+    auto copy = [=]() { std::memcpy(dst, src, n); };
     if (pageable) {   // staged before the call returns
         drain();
         copy();
@@ -143,6 +143,9 @@ int main(int argc, char** argv) {
     if (what == "no-threads" || what == "one-thread") {
         gThreads = what == "one-thread" ? 1 : 0;
         return roundTrip(cudaMemoryTypeUnregistered) ? 0 : 1;
+    }
+    if (what == "device-pointers") {   // the runtime copies or refuses them; the host cannot read them
+        return roundTrip(cudaMemoryTypeDevice) && gDirect == 2 * 6 ? 0 : 1;
     }
     return 2;
 }

@@ -20,6 +20,6 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("case", ["pageable", "pinned", "no-pinned-memory", "no-threads", "one-thread"])
+@pytest.mark.parametrize("case", ["pageable", "pinned", "no-pinned-memory", "no-threads", "one-thread", "device-pointers"])
 def test_copies(program, case):
     assert subprocess.run([program, case], timeout=60).returncode == 0

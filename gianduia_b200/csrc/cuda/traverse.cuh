@@ -647,6 +647,7 @@ __device__ __forceinline__ int traceOne(const SceneView& s, const TRay& ray, THi
 // Persistent traversal loop. Every lane of every warp runs it to the end (the block size
 // is a multiple of 32 and no lane exits early). Src provides:
 //   uint32_t count()                      number of rays
+//   kWalkNaN                              true: rays that miss everything (missesAll) are walked all the same
 //   bool load(uint32_t i, TRay&, const SceneView*&, const uint8_t*& nullMask)
 //   void world(V3& o, V3& d, float& tmin) const   the ray in flight again (leaving a mesh)
 //   void store(uint32_t i, const THit&, const SceneView&)   (the query's scene)
@@ -705,8 +706,8 @@ __device__ __forceinline__ int persistentTrace(Src& src, uint32_t* fetchCounter,
                 // a source may decline an item (it belongs to another kernel of the launch)
                 if (src.load(idx, r, sv, nm)) {
                     travInit(t, *sv, r);
-                    // the counting variants report what the traversal visits, a NaN ray's too
-                    if (!COUNT && !t.fast && missesAll(*sv, r)) t.cur = kEmpty;
+                    // counted ray batches report what the traversal visits, a NaN ray's too
+                    if (!Src::kWalkNaN && !t.fast && missesAll(*sv, r)) t.cur = kEmpty;
                     nodes = sv->nodes;
                     if (MOTION) time = r.time;
                     active = true;

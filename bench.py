@@ -191,8 +191,8 @@ def traversal_leg(ctx):
                        "(origins U[-0.5,1.5]^3, uniform directions, tmax inf)"}
     closest = lambda: ctx.trace_closest_dev(sid, dr.data_ptr(), n, dh.data_ptr(), st)
     anyhit = lambda: ctx.trace_any_dev(sid, dr.data_ptr(), n, docc.data_ptr(), st)
-    # default settings (trace_leaf_batch 12); the full node phase of every warp
-    # (trace_leaf_batch 32, the earlier default); the batch traversed in ray-key order
+    # default settings (trace_leaf_batch 12); the longest node phases (trace_leaf_batch 32,
+    # which the kernel takes as 16, a leaf pass's worth); the batch traversed in ray-key order
     # (ray_sort bit 2, the reordering inside the timed region)
     runs = [("closest", closest, {}), ("any", anyhit, {}),
             ("closest_full_node_phase", closest, {"trace_leaf_batch": 32}),
@@ -229,6 +229,8 @@ def traversal_leg(ctx):
                 "closest_achieved_gbs": achieved, "l2_read_gbs": l2, "hbm_read_gbs": hbm,
                 "scene_bytes": scene_bytes, "frac_of_l2": achieved / l2, "frac_of_hbm": achieved / hbm,
                 "bound": "l2" if scene_bytes < 100e6 else "hbm",
+                "bytes_note": "node visits and triangle tests of the plain nearest-first traversal; the timed kernel "
+                              "drops inner nodes beyond the hit, so it reads fewer bytes",
                 "hit_frac": float((dh[:, 3] >= 0).float().mean().item())})
     ctx.free_scene(sid)
     del dr, dh, docc, nodes, tris
@@ -678,8 +680,8 @@ def main():
     simt = {"node_phase": pst["extend_nodes"] / (32.0 * max(1, pst["extend_node_warp_steps"])),
             "leaf_phase": pst["extend_leaf_steps"] / (32.0 * max(1, pst["extend_leaf_warp_steps"])),
             "node_steps_per_leaf_step": pst["extend_node_warp_steps"] / max(1, pst["extend_leaf_warp_steps"]),
-            "note": "fraction of a warp's 32 lanes busy per step (node visits or leaf steps / 32 x warp steps), "
-                    "counting variant of kExtend, 8 passes with the tuned settings"}
+            "note": "fraction of a warp's 32 lanes busy per step (node visits, or triangle and instance tests, / "
+                    "32 x warp steps), counting variant of kExtend, 8 passes with the tuned settings"}
 
     peaks, peak_kind = measured_peaks()
     bytes_per_ray = nodes_per_ray * 128 + tris_per_ray * 48 + 32 + 32
@@ -711,6 +713,8 @@ def main():
                      "frac": (achieved / peaks["hbm_gbs"]) if achieved else None, "traffic": traffic,
                      "kernel": "kExtend (closest-hit BVH4 traversal)",
                      "bytes_per_ray": bytes_per_ray, "nodes_per_ray": nodes_per_ray, "tris_per_ray": tris_per_ray,
+                     "bytes_note": "the nodes that the timed kernel's own loop visits (its counting variant) and the "
+                                   "triangles it tests",
                      "launches": ext_launches, "ms_total": ext_ms, "lanes_busy": simt,
                      "peak_kind": peak_kind + " (copy bandwidth)",
                      "timed_in": "a separate instrumented render of the same %d passes (CUDA events around each "

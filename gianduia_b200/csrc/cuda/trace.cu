@@ -28,7 +28,7 @@ struct BatchSrc {
     TraceCounters* cnt;
     const uint32_t* perm;
     uint32_t cur = 0;   // the ray in flight
-    static constexpr bool kWalkNaN = COUNT;
+    static constexpr bool kPlainWalk = COUNT;
     unsigned long long sumNodes = 0, sumTris = 0;   // COUNT: this lane's rays, for the context totals
     __device__ uint32_t count() const { return n; }
     __device__ bool load(uint32_t k, TRay& r, const SceneView*& s, const uint8_t*& nm) {

@@ -42,7 +42,8 @@ __device__ __forceinline__ float lmax(float a, float b) { return a > b ? a : b; 
 
 // Work counters of the counting variants: node visits and triangle tests per lane, and
 // for the phases of the persistent loop (persistentTrace) the warp steps of each phase
-// (counted by lane 0) and the lanes' leaf steps, so that lanes busy per step = lane steps
+// (counted by lane 0; a triangle pass and a step into instances are one each) and the lanes
+// that test a triangle or an instance in them, so that lanes busy per step = lane steps
 // / (32 x warp steps).
 struct TraceCounters {
     uint32_t nodes, tris;
@@ -543,6 +544,7 @@ __device__ __forceinline__ void travTriPass(Trav& t, const SceneView* sv, bool m
     const Tri* tris = reinterpret_cast<const Tri*>(
         __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(mine ? sv->tris + first : nullptr), owner));
     float th = INFINITY, u = 0.0f, v = 0.0f;
+    if (COUNT && busy) cnt->leafSteps++;
     if (busy) {
         float tt;
         uint32_t prim;
@@ -647,7 +649,8 @@ __device__ __forceinline__ int traceOne(const SceneView& s, const TRay& ray, THi
 // Persistent traversal loop. Every lane of every warp runs it to the end (the block size
 // is a multiple of 32 and no lane exits early). Src provides:
 //   uint32_t count()                      number of rays
-//   kWalkNaN                              true: rays that miss everything (missesAll) are walked all the same
+//   kPlainWalk                            true: what the plain traversal visits is visited (and counted): no
+//                                         distance check at the pop, rays that miss everything walked too
 //   bool load(uint32_t i, TRay&, const SceneView*&, const uint8_t*& nullMask)
 //   void world(V3& o, V3& d, float& tmin) const   the ray in flight again (leaving a mesh)
 //   void store(uint32_t i, const THit&, const SceneView&)   (the query's scene)
@@ -669,9 +672,9 @@ constexpr int kRefill = 8;
 template <int BLOCK, bool ANY, bool COUNT, int SMEM = kSmemStack, bool MOTION = false, bool SLOT_ORDER_ANY = false, typename Src>
 __device__ __forceinline__ int persistentTrace(Src& src, uint32_t* fetchCounter, TEntry<!ANY>* smemStack, uint32_t* smemMap,
                                                TraceCounters* cnt, uint32_t leafBatch = 32) {
-    constexpr bool kCull = !ANY && !COUNT;   // the counting variants count the plain traversal's visits
+    constexpr bool kCull = !ANY && !Src::kPlainWalk;
     // a leaf pass takes 32 triangles: waiting for more than kPassLanes lanes gains nothing
-    if (!COUNT) leafBatch = min(leafBatch, (uint32_t)kPassLanes);
+    leafBatch = min(leafBatch, (uint32_t)kPassLanes);
     TStack<BLOCK, SMEM, !ANY> st;
     st.smem = smemStack + threadIdx.x;
     uint32_t* map = smemMap + (threadIdx.x & ~31u);
@@ -706,8 +709,7 @@ __device__ __forceinline__ int persistentTrace(Src& src, uint32_t* fetchCounter,
                 // a source may decline an item (it belongs to another kernel of the launch)
                 if (src.load(idx, r, sv, nm)) {
                     travInit(t, *sv, r);
-                    // counted ray batches report what the traversal visits, a NaN ray's too
-                    if (!Src::kWalkNaN && !t.fast && missesAll(*sv, r)) t.cur = kEmpty;
+                    if (!Src::kPlainWalk && !t.fast && missesAll(*sv, r)) t.cur = kEmpty;
                     nodes = sv->nodes;
                     if (MOTION) time = r.time;
                     active = true;
@@ -739,9 +741,10 @@ __device__ __forceinline__ int persistentTrace(Src& src, uint32_t* fetchCounter,
         // leaf pass
         const bool held = t.leaf != kEmpty;
         const bool tri = held && t.curInst >= 0;
-        if (COUNT && __any_sync(0xffffffffu, held)) {
-            if ((threadIdx.x & 31) == 0) cnt->leafWarpSteps++;
-            if (held) cnt->leafSteps++;
+        if (COUNT) {   // the triangle pass counts its own lanes
+            const bool anyTri = __any_sync(0xffffffffu, tri), anyInst = __any_sync(0xffffffffu, held && !tri);
+            if ((threadIdx.x & 31) == 0) cnt->leafWarpSteps += (anyTri ? 1u : 0u) + (anyInst ? 1u : 0u);
+            if (held && !tri) cnt->leafSteps++;
         }
         if (__any_sync(0xffffffffu, tri)) travTriPass<ANY, COUNT>(t, sv, tri, map, cnt);
         if (held && !tri) {

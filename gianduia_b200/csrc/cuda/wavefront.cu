@@ -875,7 +875,7 @@ struct ExtendSrc {
     uint32_t slot;
     int32_t medium;
     bool vol;
-    static constexpr bool kWalkNaN = false;   // one such path of a large scene would take the kernel seconds
+    static constexpr bool kPlainWalk = false;   // counting renders count what renders do
     __device__ uint32_t count() const { return n; }
     __device__ bool load(uint32_t i, TRay& r, const SceneView*& sv, const uint8_t*& nm) {
         slot = p->extList[i];
@@ -1309,7 +1309,7 @@ struct ShadowSrc {
     uint32_t n;
     bool mixed;
     uint32_t rec;   // the shadow record of the query in flight (its path slot and job are read again at the store)
-    static constexpr bool kWalkNaN = false;
+    static constexpr bool kPlainWalk = false;
     __device__ uint32_t count() const { return n; }
     __device__ bool load(uint32_t i, TRay& r, const SceneView*& sv, const uint8_t*& nmOut) {
         rec = p->shadowOrder ? p->shadowOrder[i] : i;

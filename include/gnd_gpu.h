@@ -233,8 +233,9 @@ gnd_status gnd_gpu_trace_closest_dev(gnd_gpu_ctx* ctx, gnd_scene_id scene, const
                                      gnd_hit* d_hits, void* stream);
 gnd_status gnd_gpu_trace_any_dev(gnd_gpu_ctx* ctx, gnd_scene_id scene, const gnd_ray* d_rays, int64_t n,
                                  uint8_t* d_occluded, void* stream);
-/* Per-ray traversal work of the closest-hit kernel (instrumented variant): node visits
- * and triangle tests, DEVICE buffers. Used for the roofline byte counts. */
+/* Per-ray traversal work of a closest-hit query: node visits and triangle tests of the plain
+ * nearest-first traversal (instrumented variant; the closest-hit kernel itself visits fewer
+ * nodes, since it drops inner nodes beyond the hit from its stack), DEVICE buffers. */
 gnd_status gnd_gpu_trace_count_dev(gnd_gpu_ctx* ctx, gnd_scene_id scene, const gnd_ray* d_rays, int64_t n,
                                    uint32_t* d_nodes, uint32_t* d_tris, void* stream);
 /* gnd_gpu_trace_closest without any device allocation. No counterpart in the reference.
@@ -322,15 +323,15 @@ typedef struct gnd_render_stats {
     double ms;                /* device time of the render */
     int64_t extend_rays;      /* closest-hit queries of the extend kernel */
     int64_t shadow_rays;      /* shadow queries */
-    int64_t extend_nodes;     /* profile bit1: BVH4 node visits in extend */
-    int64_t extend_tris;      /* profile bit1: triangle tests in extend */
+    int64_t extend_nodes;     /* profile bit1: BVH4 node visits of the extend kernel's traversal */
+    int64_t extend_tris;      /* profile bit1: its triangle tests */
     double extend_ms;         /* profile bit0: summed device time of the extend launches */
     int64_t iterations;       /* wavefront iterations (bounce steps) */
     int64_t launches;         /* kernels the render launched */
     /* profile bit1: the extend traversal's phases (a warp alternates inner-node steps and
-     * leaf steps): warp steps of the node phase, lane steps and warp steps of the leaf
-     * phase; lanes busy per step = extend_nodes / (32 x extend_node_warp_steps) and
-     * extend_leaf_steps / (32 x extend_leaf_warp_steps) */
+     * leaf steps): warp steps of the node phase; lanes that test a triangle or an instance
+     * and warp steps of the leaf phase; lanes busy per step = extend_nodes /
+     * (32 x extend_node_warp_steps) and extend_leaf_steps / (32 x extend_leaf_warp_steps) */
     int64_t extend_node_warp_steps;
     int64_t extend_leaf_steps;
     int64_t extend_leaf_warp_steps;

@@ -2781,7 +2781,13 @@ gnd_status gnd_gpu_autotune(gnd_gpu_ctx* ctxh, gnd_scene_id id, int32_t spp, int
             {&Tune::travBlocks, {8, 6, 4}}, {&Tune::smem, {32, 16}},          {&Tune::sort, {1, 0}},
             {&Tune::poolLog2, {22, 21, 23, 24, 20}}, {&Tune::roundIters, {8, 16, 4}}, {&Tune::graphs, {1, 0}},
             {&Tune::sampleFilm, {1, 0}},
-            {&Tune::raySort, {1, 3, 0}}, {&Tune::leafBatch, {16, 8, 24, 32}}, {&Tune::shadowLeafBatch, {16, 8, 24, 32}},
+            {&Tune::raySort, {1, 3, 0}}, {&Tune::leafBatch, {32, 8}}, {&Tune::shadowLeafBatch, {32, 8}},
+        };
+        // Two values of a setting that run the same code: the leaf batches above kPassLanes. Timed
+        // against each other they would be told apart by noise alone.
+        auto same = [](int Tune::*field, int a, int b) {
+            if (field == &Tune::leafBatch || field == &Tune::shadowLeafBatch) return std::min(a, kPassLanes) == std::min(b, kPassLanes);
+            return a == b;
         };
         for (int sweep = 0; sweep < 2; ++sweep) {
             bool changed = false;
@@ -2790,7 +2796,7 @@ gnd_status gnd_gpu_autotune(gnd_gpu_ctx* ctxh, gnd_scene_id id, int32_t spp, int
                     if (spentMs() > budgetMs) break;
                     // the render knobs only: ray_sort keeps its ray-batch bit (bit 2)
                     const int value = k.field == &Tune::raySort ? (v | (cur.raySort & 4)) : v;
-                    if (cur.*(k.field) == value) continue;
+                    if (same(k.field, cur.*(k.field), value)) continue;
                     Tune t = cur;
                     t.*(k.field) = value;
                     double m = trial(t);

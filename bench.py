@@ -479,8 +479,8 @@ def serve_leg(ctx, microfacet_sid, n_requests, n_policy=300):
             "deadline_p50_s": other["deadline"]["p50"], "deadline_p99_s": other["deadline"]["p99"],
             "plain_model": model,
             "note": "plain time-to-image: the FIFO recurrence over plain render times, each the fixed + spp x "
-                    "per-pass time measured for its (scene, resolution, depth) (plain renders run their passes "
-                    "one after another); served_mpaths_s at 80% offered load is bounded by the arrivals"}
+                    "per-pass time of its (scene, resolution, depth), measured with 4 and 16 passes; "
+                    "served_mpaths_s at 80% offered load is bounded by the arrivals"}
 
 
 def main():

@@ -4,14 +4,14 @@
 
   served : every request is submitted to the context's job server (gnd_gpu_serve_*) at
            its arrival time; jobs share one pool of path slots, oldest job first.
-  plain  : one request at a time through gnd_gpu_render (one sample pass in flight),
-           first come first served. Its time-to-image follows from each request's
+  plain  : one request at a time through gnd_gpu_render (passes handed out one after
+           another), first come first served. Its time-to-image follows from each request's
            render time by the single-server FIFO recurrence
            finish_i = max(arrival_i, finish_{i-1}) + service_i. The render time is
            measured per request (run_plain_service) or, for long streams, modelled from
-           measured renders (plain_service_model): a plain render runs its passes one
-           after another, so its time is a fixed part plus spp times a per-pass part,
-           both measured for every (scene, resolution, depth) of the stream.
+           measured renders (plain_service_model): from some passes on, a plain render's
+           time grows by the same time per pass, so it is a fixed part plus spp times a
+           per-pass part, both measured for every (scene, resolution, depth) of the stream.
 
 Per request, uniformly: scene, square resolution in {128, 256, 512, 1024}, spp in
 {4, 16, 64}, maximum depth in 8..32. Time-to-image runs from arrival to the finished
@@ -131,21 +131,23 @@ def _plain_time(ctx, sid, integrator, res, spp, depth):
 
 
 def plain_service_model(ctx, sids, integrators, reqs, check=6):
-    """Plain (one pass in flight) render times of the requests without rendering each one:
-    for every distinct (scene, resolution, depth) of the stream a 1-pass and a 4-pass
-    plain render are timed (host wall time, as run_plain_service), giving
-    time(spp) = fixed + spp * per_pass with per_pass = (t4 - t1) / 3. `check` requests of
-    spp 16 or 64 are also rendered in full and compared with the model.
+    """Plain render times of the requests without rendering each one: for every distinct
+    (scene, resolution, depth) of the stream a 4-pass and a 16-pass plain render are timed
+    (host wall time, as run_plain_service), giving time(spp) = fixed + spp * per_pass with
+    per_pass = (t16 - t4) / 12. A pass begins while the last paths of the one before finish,
+    so the first passes are not representative (fitted to 1 and 4 passes, 16- and 64-pass
+    renders come out 12% too low or too high; to 4 and 16 passes, 64-pass ones within 6%). `check`
+    requests of spp 16 or 64 are also rendered in full and compared with the model.
     Returns (service times in s, dict with the model's size and its largest relative error)."""
     keys = sorted({(r["scene"], r["res"], r["max_depth"]) for r in reqs})
     model = {}
     for sc, res, depth in keys:
         sid, integ = sids[sc], integrators[sc]
         _plain_time(ctx, sid, integ, res, 1, depth)   # warm-up (first use of this film size)
-        t1 = _plain_time(ctx, sid, integ, res, 1, depth)
         t4 = _plain_time(ctx, sid, integ, res, 4, depth)
-        per = max((t4 - t1) / 3.0, 0.0)
-        model[(sc, res, depth)] = (max(t1 - per, 0.0), per)
+        t16 = _plain_time(ctx, sid, integ, res, 16, depth)
+        per = max((t16 - t4) / 12.0, 0.0)
+        model[(sc, res, depth)] = (t4 - 4.0 * per, per)
 
     def predict(r):
         fixed, per = model[(r["scene"], r["res"], r["max_depth"])]

@@ -13,7 +13,17 @@ namespace gnd {
 
 Server::Server(Context* c) : c_(c), t0_(std::chrono::steady_clock::now()) {
     thread_ = std::thread([this]() { loop(); });
-    finisher_ = std::thread([this]() { finishLoop(); });
+    try {
+        finisher_ = std::thread([this]() { finishLoop(); });
+    } catch (...) {   // no second thread: the first must end before the members go
+        {
+            std::lock_guard<std::mutex> lk(m_);
+            stop_ = true;
+        }
+        workCv_.notify_all();
+        thread_.join();
+        throw;
+    }
 }
 
 Server::~Server() {

@@ -1070,7 +1070,11 @@ __global__ void __launch_bounds__(kAggBlock, 4) kClassify(KParams p, uint32_t* c
 // class (medium sampling marked done) for a surface kernel later in the iteration.
 // EXT: some job of the launch uses the rarer features (SceneView::ext); without them the
 // kernel keeps the area-light, static-transform code only.
-// 128 registers (4 blocks per SM); the all-lobe kernels, which few paths take, up to 255.
+// 128 registers (4 blocks per SM); the all-lobe kernels, which few paths take, up to 255. The EXT
+// kernels want 168 and spill 260 to 416 bytes at 128, and are faster for it all the same: 512^2 x
+// 16 renders at 3 | 4 blocks: environment map 3.11 | 3.08 ms, point, spot and directional lights
+// 2.41 | 2.42, environment and point light in volpath 3.18 | 3.13, moving boxes 10.82 | 10.50,
+// thin lens 8.07 | 7.71, texture trees 10.33 | 10.07, with normal and bump maps 13.05 | 12.24.
 template <bool VOL, uint32_t M, bool EXT>
 __global__ void __launch_bounds__(kBlock, M == kLobesAll ? 2 : 4) kShade(KParams p, const uint32_t* list, const uint32_t* count) {
     const uint32_t n = *count;
@@ -2061,25 +2065,6 @@ uint64_t Wavefront::retired(int j) {
     GND_CUDA(cudaStreamSynchronize(ctx_->stream));
     jobs_[j].retired = c.retired;
     return c.retired;
-}
-
-void Wavefront::readRetired(std::vector<uint64_t>& out) {
-    JobCtl c[kMaxJobs];
-    GND_CUDA(cudaMemcpyAsync(c, ctl_.ptr, sizeof(c), cudaMemcpyDeviceToHost, ctx_->stream));
-    GND_CUDA(cudaStreamSynchronize(ctx_->stream));
-    out.resize(kMaxJobs);
-    for (int j = 0; j < kMaxJobs; ++j) {
-        out[j] = c[j].retired;
-        if (jobs_[j].used) jobs_[j].retired = c[j].retired;
-    }
-}
-
-void Wavefront::readCtl(std::vector<JobCtl>& out) {
-    out.resize(kMaxJobs);
-    GND_CUDA(cudaMemcpyAsync(out.data(), ctl_.ptr, kMaxJobs * sizeof(JobCtl), cudaMemcpyDeviceToHost, ctx_->stream));
-    GND_CUDA(cudaStreamSynchronize(ctx_->stream));
-    for (int j = 0; j < kMaxJobs; ++j)
-        if (jobs_[j].used) jobs_[j].retired = out[j].retired;
 }
 
 void Wavefront::useSampleRecords(int j, uint64_t items) {

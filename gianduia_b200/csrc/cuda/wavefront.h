@@ -157,8 +157,6 @@ public:
     void enqueueRound(int iters, int integratorMix, bool hasNull, int profile, Result& acc, int slot);
     const Snapshot& waitRound(int slot);
     uint64_t retired(int job);                        // reads the job's retired count (sync)
-    void readRetired(std::vector<uint64_t>& out);     // all jobs (one copy, sync)
-    void readCtl(std::vector<JobCtl>& out);           // all jobs' hand-out and retired counts (sync)
     // Gives the job a per-sample record buffer for `items` work items (see JobDev::samples);
     // filmFromSamples() then adds the records into the job's film.
     void useSampleRecords(int job, uint64_t items);

@@ -136,7 +136,7 @@ def plain_service_model(ctx, sids, integrators, reqs, check=6):
     (host wall time, as run_plain_service), giving time(spp) = fixed + spp * per_pass with
     per_pass = (t16 - t4) / 12. A pass begins while the last paths of the one before finish,
     so the first passes are not representative (fitted to 1 and 4 passes, 16- and 64-pass
-    renders come out 12% too low or too high; to 4 and 16 passes, 64-pass ones within 6%). `check`
+    renders come out 12% too low or too high; to 4 and 16 passes, 64-pass ones within 7%). `check`
     requests of spp 16 or 64 are also rendered in full and compared with the model.
     Returns (service times in s, dict with the model's size and its largest relative error)."""
     keys = sorted({(r["scene"], r["res"], r["max_depth"]) for r in reqs})
@@ -157,6 +157,8 @@ def plain_service_model(ctx, sids, integrators, reqs, check=6):
     errs = []
     big = [r for r in reqs if r["spp"] >= 16][:check]
     for r in big:
+        # as for the model: a scene with other engine settings before it dropped the graphs
+        _plain_time(ctx, sids[r["scene"]], integrators[r["scene"]], r["res"], 1, r["max_depth"])
         meas = _plain_time(ctx, sids[r["scene"]], integrators[r["scene"]], r["res"], r["spp"], r["max_depth"])
         errs.append(abs(predict(r) - meas) / meas)
     return svc, {"keys": len(keys), "checked": len(errs), "max_rel_err": float(max(errs)) if errs else None}

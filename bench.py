@@ -491,7 +491,7 @@ def main():
     ap.add_argument("--impl", default="gpu", choices=["gpu", "reference"])
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")
-    ap.add_argument("--plain", action="store_true", help="one pass in flight (no refill) for the timed steps")
+    ap.add_argument("--plain", action="store_true", help="plain renders (a pool of one pass, passes handed out one after another) for the timed steps")
     ap.add_argument("--no-traversal", action="store_true", help="skip the traversal micro-benchmark")
     ap.add_argument("--no-autotune", action="store_true", help="render with the default engine settings")
     ap.add_argument("--no-scenes", action="store_true", help="skip the Cornell / volumetric renders")
@@ -703,7 +703,7 @@ def main():
         "data": "synthetic (seeded generator, gianduia_b200/scenes.py)",
         "config": {"workload": "microfacet 1024x1024, 64 spp, path_gpu depth 16, 5,242,882 tris, 4105 instances, 8 sphere lights",
                    "parallelism": "spp-sharded" if world > 1 else "single GPU",
-                   "mode": "batched (all passes share a refilled pool of path slots)" if batched else "plain (one pass in flight)",
+                   "mode": "batched (all passes share a refilled pool of path slots)" if batched else "plain (a pool of one pass, passes handed out one after another)",
                    "l2": "inputs larger than L2 (scene %.2f GB resident)" % (scene_bytes / 1e9),
                    "graphs": "per-bounce loop replayed as CUDA graphs" if tune.get("graphs") else "graphs off",
                    "tune": tune},

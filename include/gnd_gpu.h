@@ -305,8 +305,11 @@ typedef struct gnd_render_params {
     int32_t max_depth;        /* <= 0: the scene file's value */
     int32_t integrator;       /* -1: the scene file's; 0 path_gpu; 1 volpath_gpu */
     int32_t window[4];        /* pixel window x0, y0, x1, y1; all zero: the full image */
-    int32_t batched;          /* 0: one pass in flight at a time (plain); 1: every pass
-                                 shares the path pool, refilled as paths finish */
+    int32_t batched;          /* 0 (plain): a pool of one pass's paths, passes handed out
+                                 whole, one after another; without a callback the next
+                                 begins as paths of the last one end, with a callback when
+                                 the last one has ended; 1: every pass shares the path
+                                 pool, refilled as paths finish */
     int32_t profile;          /* bit0: time the closest-hit (extend) launches with events;
                                  bit1: count BVH node visits / triangle tests in extend */
     gnd_progress_fn callback; /* optional (plain mode only) */

@@ -663,7 +663,8 @@ __device__ __forceinline__ int traceOne(const SceneView& s, const TRay& ray, THi
 // `map`: 32 words of shared memory per warp.
 // Measured (one B200; 4.2M random rays on 2^20 triangles / 32 passes of the 1024^2 sphere grid):
 // full node phases, refill of any idle lane 2.30 ms / 101.6 ms, one child per step, triangle by
-// triangle; this loop 1.77 / 88.5. Its parts: kPassLanes 32, 24, 16, 12: - / 98.9, 95.3, 94.1,
+// triangle; this loop 1.77 / 88.5 while it dropped leaves beyond the hit as well (1% more
+// without, see cullKey). Its parts: kPassLanes 32, 24, 16, 12: - / 98.9, 95.3, 94.1,
 // 95.9; kRefill 1, 4, 8, 12: 1.94, 1.90, 1.88, 1.94 / -, 93.0, 91.5, -; child references loaded
 // with the boxes instead of after the sort -4% / -0.7%; reciprocals kept across a translation
 // -1.5% / -2%. Two steps per vote, 7 or 6 blocks per SM: no gain on the small scenes.

@@ -1368,7 +1368,7 @@ __global__ void __launch_bounds__(kBlock, kTravBlocks) kShadowPath(KParams p, bo
 // Shadow queries of `volpath`: evaluateTr (volPath.cpp:261-291), a loop of closest hits
 // through null-BSDF boundaries multiplying the transmittance of each medium segment.
 // 8, 6, 4 blocks per SM (64 registers with spills .. 127 without): 5.8, 6.0, 5.9 ms of the
-// volumetric 512^2 x 16 render; 8.1 ms with a stack of every child and unpacked arithmetic.
+// volumetric 512^2 x 16 render (6.0 at 8 blocks since leaves beyond the hit are tested); 8.1 ms with a stack of every child and unpacked arithmetic.
 template <bool MOTION>
 __global__ void __launch_bounds__(kBlock, 8) kShadow(KParams p, bool mixed) {
     __shared__ TEntry<true> stack[kSmemStack * kBlock];

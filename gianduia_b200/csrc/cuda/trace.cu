@@ -139,14 +139,30 @@ namespace {
 // Batches of at least this many rays are reordered when the scene's ray_sort has bit 2.
 constexpr int64_t kBatchSortMin = 1 << 16;
 
+// Blocks of a batch of n rays, at most bps per SM. Small batches are spread over all warps (a
+// warp per ray, then a few rays each: persistentTrace): a warp's steps grow with the number of
+// its rays that diverge, and the warps are there. From some rays a warp on, the warps' own
+// instructions cost more than that saves, sooner in a small tree, whose rays take few and
+// similar steps; the batch then goes 32 rays a warp to as many blocks as that takes, which the
+// hardware deals out evenly over the SMs. Closest hit, us, 32 rays a warp from the start | always
+// spread | by this rule, 19000, 38000 and 90000 rays: Cornell box (4 nodes) 32, 34, 40 | 33, 37,
+// 43 | 28, 29, 36; 800 triangles 38, 40, 47 | 32, 37, 45 | 30, 33, 40; 2^18 triangles 215, 220, 268
+// | 124, 150, 193 | 123, 153, 187.
+constexpr int64_t kSmallTree = 4096;   // nodes
+int traceGrid(const Context* c, const DeviceScene& ds, int64_t n, int bps) {
+    constexpr int64_t kWarps = kTraceBlock / 32;
+    const int64_t most = (int64_t)c->numSMs * bps;
+    const int64_t spread = most * kWarps * (ds.numNodes < kSmallTree ? 4 : 8);
+    const int64_t blocks = n <= spread ? (n + kWarps - 1) / kWarps : (n + kTraceBlock - 1) / kTraceBlock;
+    return (int)std::max<int64_t>(1, std::min(blocks, most));
+}
+
 void launchTrace(Context* c, DeviceScene& ds, const gnd_ray* dr, int64_t n, gnd_hit* dh, uint8_t* docc,
                  uint32_t* dn, uint32_t* dt, cudaStream_t st) {
     if (n <= 0) return;
     if (n >= (int64_t)0xF0000000LL) throw Error(GND_ERR_INVALID, "ray batch too large (limit 4e9 rays per call)");
-    // small batches: a warp per ray as long as the grid has room (persistentTrace spreads them)
-    int64_t blocks = (n + kTraceBlock / 32 - 1) / (kTraceBlock / 32);
     const int bps = std::min(std::max(ds.tune.traceBlocks, 1), kTraceBlocksPerSM);
-    int g = (int)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)c->numSMs * bps));
+    const int g = traceGrid(c, ds, n, bps);
     uint32_t* ew = c->errWord.as<uint32_t>();
     uint32_t* fetch = c->nextFetchCounter();
     GND_CUDA(cudaMemsetAsync(fetch, 0, sizeof(uint32_t), st));
@@ -309,8 +325,7 @@ gnd_status gnd_gpu_trace_closest_fixed(gnd_gpu_ctx* ctxh, gnd_scene_id id, const
         cudaStream_t st = c->stream;
         GND_CUDA(cudaMemcpyAsync(dr, rays, sizeof(gnd_ray) * (size_t)n, cudaMemcpyHostToDevice, st));
         GND_CUDA(cudaMemsetAsync(fetch, 0, sizeof(uint32_t), st));
-        int64_t blocks = (n + kTraceBlock / 32 - 1) / (kTraceBlock / 32);
-        int g = (int)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)c->numSMs * kTraceBlocksPerSM));
+        const int g = traceGrid(c, ds, n, kTraceBlocksPerSM);
         traceKernel<false, false><<<g, kTraceBlock, 0, st>>>(ds.viewDev.as<SceneView>(), dr, (uint32_t)n, dh, nullptr,
                                                              nullptr, nullptr, fetch, c->errWord.as<uint32_t>(),
                                                              c->traceTotals.as<unsigned long long>(), nullptr, 32u);
